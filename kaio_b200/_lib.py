@@ -1,4 +1,7 @@
-"""ctypes loader for ``libkaio_b200.so`` -- the only route from Python to the kernels.
+"""Loaders of ``libkaio_b200.so`` (ctypes) and of the extension module ``_native`` that calls it.
+
+The ops go through ``_native``: one C call per op, arguments unpacked in C++ (12-16 us of host time
+per call with ctypes, below 5 us this way).  ctypes serves the queries that are not on a hot path.
 
 There is no fallback: when the shared library is missing, loading raises; when the machine has
 no sm_100 GPU, every op returns an error code that ``ops`` turns into ``KaioError``.
@@ -92,3 +95,23 @@ def load() -> C.CDLL:
     lib.kaio_b200_version.argtypes = []
     _lib = lib
     return lib
+
+
+class _Native:
+    """``kaio_b200/_native.so``, imported at the first use of one of its functions."""
+
+    def __getattr__(self, name):
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        if not os.path.exists(LIB_PATH):
+            load()  # raises
+        try:
+            from . import _native
+        except ImportError as e:
+            raise RuntimeError(f"the extension module kaio_b200._native is missing or does not load ({e}): build it "
+                               "with `python -m kaio_b200.build`") from e
+        fn = getattr(_native, name)
+        setattr(self, name, fn)  # later look-ups do not come here
+        return fn
+
+
+native = _Native()

@@ -4,7 +4,9 @@ Run as ``python -m kaio_b200.build`` or through ``__graft_entry__.build()``.  nv
 cross-compiles without a GPU.  Each ``csrc/*.cu`` is compiled to an object in parallel and
 linked into ``kaio_b200/lib/libkaio_b200.so``; the CUDA runtime is linked statically and the
 driver API is reached through the runtime's entry-point lookup, so the library loads on a
-machine without ``libcuda.so`` (where every op then reports a CUDA error).
+machine without ``libcuda.so`` (where every op then reports a CUDA error).  ``csrc/bindings.cpp``
+(the argument unpacking of ``kaio_b200.ops``) becomes the extension module ``kaio_b200/_native.so``,
+linked against that library.
 """
 from __future__ import annotations
 
@@ -14,12 +16,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(LIB_DIR, "libkaio_b200.so")
+NATIVE = os.path.join(HERE, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -78,7 +82,29 @@ def build(force: bool = False, verbose: bool = False) -> str:
                             "-gencode", "arch=compute_100a,code=sm_100a"], capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_native(force)
     return LIB
+
+
+def build_native(force: bool = False) -> str:
+    """Compiles ``csrc/bindings.cpp`` against the installed torch and this library."""
+    import importlib.util
+    src = os.path.join(CSRC, "bindings.cpp")
+    header = os.path.join(os.path.dirname(HERE), "include", "kaio_b200.h")
+    if not force and os.path.exists(NATIVE) and \
+            os.path.getmtime(NATIVE) >= max(os.path.getmtime(src), os.path.getmtime(header)):
+        return NATIVE
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    inc = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include/torch/csrc/api/include"),
+           sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    r = subprocess.run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+                        *[f"-I{d}" for d in inc], src, "-o", NATIVE, f"-L{LIB_DIR}", "-lkaio_b200",
+                        f"-L{os.path.join(torch_dir, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+                        "-Wl,-rpath,$ORIGIN/lib"], capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {src}:\n{r.stdout}\n{r.stderr}")
+    return NATIVE
 
 
 if __name__ == "__main__":
