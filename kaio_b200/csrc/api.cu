@@ -962,6 +962,8 @@ KAIO_API int32_t kaio_b200_attention_tc(const kaio_f16* q, size_t q_len, const k
     p.causal = causal ? 1 : 0;
     p.out_f16 = 0;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (attention_decode_ok(p))
+        return finish(launch_attention_decode(*ctx, p, s), "attention_tc", "attention_decode");
     if (flash_attention_ok(p))
         return finish(launch_flash_attention(*ctx, p, s), "attention_tc", "flash_tcgen05");
     return finish(launch_attention_generic(p, s), "attention_tc", "attention_generic");
@@ -984,8 +986,6 @@ KAIO_API int32_t kaio_b200_attention_mha_f16(const kaio_f16* q, size_t q_len, co
     if (head_dim > 256)
         return fail(KAIO_B200_ERR_INVALID_CONFIG, "%s: head_dim must be \xE2\x89\xA4 256 (got %u)",
                     op, head_dim);
-    if (attention_decode_ok(p))
-        return finish(launch_attention_decode(*ctx, p, s), "attention_tc", "attention_decode");
     const size_t need_q = ((size_t)batch * seq_q - 1) * row_stride + (size_t)heads * head_dim;
     const size_t need_k = ((size_t)batch * seq_k - 1) * row_stride + (size_t)heads * head_dim;
     if (q_len < need_q)
@@ -1026,6 +1026,8 @@ KAIO_API int32_t kaio_b200_attention_mha_f16(const kaio_f16* q, size_t q_len, co
     p.causal = causal ? 1 : 0;
     p.out_f16 = 1;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (attention_decode_ok(p))
+        return finish(launch_attention_decode(*ctx, p, s), op, "attention_decode");
     if (flash_attention_ok(p))
         return finish(launch_flash_attention(*ctx, p, s), op, "flash_tcgen05");
     return finish(launch_attention_generic(p, s), op, "attention_generic");
@@ -1048,8 +1050,6 @@ KAIO_API int32_t kaio_b200_quantize_rows_int8(const float* x, size_t x_len, int8
         return fail(KAIO_B200_ERR_INVALID_CONFIG,
                     "%s: Q buffer too small: need %zu i8 (%u\xC3\x97%u), got %zu", op, mk, m, k,
                     q_len);
-    if (attention_decode_ok(p))
-        return finish(launch_attention_decode(*ctx, p, s), op, "attention_decode");
     if (scale_len < m)
         return fail(KAIO_B200_ERR_INVALID_CONFIG,
                     "%s: scale buffer too small: need %u f32, got %zu", op, m, scale_len);

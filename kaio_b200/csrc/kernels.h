@@ -196,10 +196,10 @@ struct AttnParams {
 };
 
 cudaError_t launch_attention_generic(const AttnParams& p, cudaStream_t stream);
+// One query row per (batch, head), head_dim 64 or 128: the key range of a pair over a cluster.
+bool attention_decode_ok(const AttnParams& p);
+cudaError_t launch_attention_decode(const DeviceCtx& ctx, const AttnParams& p, cudaStream_t stream);
 bool flash_attention_ok(const AttnParams& p);
 cudaError_t launch_flash_attention(const DeviceCtx& ctx, const AttnParams& p, cudaStream_t stream);
 
 }  // namespace kaio
-// One query row per (batch, head), head_dim 64 or 128: the key range of a pair over a cluster.
-bool attention_decode_ok(const AttnParams& p);
-cudaError_t launch_attention_decode(const DeviceCtx& ctx, const AttnParams& p, cudaStream_t stream);
