@@ -514,6 +514,18 @@ static uint32_t fused_max_m()
     return v;
 }
 
+// Largest M the fused W8A16 kernel takes: up to 256 rows one tile holds them all and every weight is
+// converted once.  KAIO_B200_W8A16_FUSED_MAX_M overrides it (tuning aid).
+static uint32_t w8a16_fused_max_m()
+{
+    static const uint32_t v = [] {
+        if (const char* e = getenv("KAIO_B200_W8A16_FUSED_MAX_M"))
+            return (uint32_t)strtoul(e, nullptr, 10);
+        return 256u;
+    }();
+    return v;
+}
+
 static int32_t run_int4(const kaio_f16* a, size_t a_len, const uint32_t* b, size_t b_len,
                         const kaio_f16* scales, size_t s_len, void* c, size_t c_len, bool out_f16,
                         uint32_t m, uint32_t n, uint32_t k, uint32_t group_size, void* stream)
@@ -590,6 +602,9 @@ static int32_t run_qkv(int wfmt, const char* op, const __half* x, DqProblem prob
                                          ws ? sc->tile_counters : nullptr, s),
                       op, ws ? "qkv_w4a16_fused_dequant_splitk" : "qkv_w4a16_fused_dequant");
     }
+    if (wfmt == WFMT_S8_ROWMAJOR && post_scale && m <= w8a16_fused_max_m() &&
+        w8a16_fused_ok(x, probs, 3, m, n, k))
+        return finish(launch_w8a16_fused(*ctx, x, probs, 3, m, n, k, s), op, "qkv_w8a16_fused");
     if (dq_gemm_fast_path_ok(wfmt, x, probs, 3, true, m, n, k)) {
         if ((rc = ensure_dq_workspace(ctx, s, dq_gemm_workspace_bytes(3, n, k), &sc)))
             return rc;

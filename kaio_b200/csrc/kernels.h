@@ -98,6 +98,13 @@ cudaError_t launch_w4a16_fused(const DeviceCtx& ctx, const __half* x, const DqPr
                                void* workspace, uint32_t* counters, cudaStream_t stream,
                                const OutputCopies* copies = nullptr);
 
+// Fused W8A16 GEMM for few rows (f16 out, post-scale): s8 -> f16 inside the GEMM.
+bool w8a16_fused_ok(const void* x, const DqProblem* probs, int num_probs, uint32_t m, uint32_t n,
+                    uint32_t k);
+cudaError_t launch_w8a16_fused(const DeviceCtx& ctx, const __half* x, const DqProblem* probs,
+                               int num_probs, uint32_t m, uint32_t n, uint32_t k,
+                               cudaStream_t stream);
+
 bool dq_gemm_fast_path_ok(int wfmt, const void* x, const DqProblem* probs, int num_probs,
                           bool out_f16, uint32_t m, uint32_t n, uint32_t k);
 // Destinations of a single-output GEMM: the [m, n] result is stored to every ptrs[r] (already
