@@ -979,6 +979,8 @@ KAIO_API int32_t kaio_b200_attention_tc(const kaio_f16* q, size_t q_len, const k
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (attention_decode_ok(p))
         return finish(launch_attention_decode(*ctx, p, s), "attention_tc", "attention_decode");
+    if (attention_warp_ok(*ctx, p))
+        return finish(launch_attention_warp(*ctx, p, s), "attention_tc", "attention_warp_mma");
     if (flash_attention_ok(p))
         return finish(launch_flash_attention(*ctx, p, s), "attention_tc", "flash_tcgen05");
     return finish(launch_attention_generic(p, s), "attention_tc", "attention_generic");
@@ -1043,6 +1045,8 @@ KAIO_API int32_t kaio_b200_attention_mha_f16(const kaio_f16* q, size_t q_len, co
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (attention_decode_ok(p))
         return finish(launch_attention_decode(*ctx, p, s), op, "attention_decode");
+    if (attention_warp_ok(*ctx, p))
+        return finish(launch_attention_warp(*ctx, p, s), op, "attention_warp_mma");
     if (flash_attention_ok(p))
         return finish(launch_flash_attention(*ctx, p, s), op, "flash_tcgen05");
     return finish(launch_attention_generic(p, s), op, "attention_generic");

@@ -206,6 +206,9 @@ cudaError_t launch_attention_generic(const AttnParams& p, cudaStream_t stream);
 // One query row per (batch, head), head_dim 64 or 128: the key range of a pair over a cluster.
 bool attention_decode_ok(const AttnParams& p);
 cudaError_t launch_attention_decode(const DeviceCtx& ctx, const AttnParams& p, cudaStream_t stream);
+// Warp-level MMAs: head_dim 64, and short sequences of few heads.
+bool attention_warp_ok(const DeviceCtx& ctx, const AttnParams& p);
+cudaError_t launch_attention_warp(const DeviceCtx& ctx, const AttnParams& p, cudaStream_t stream);
 bool flash_attention_ok(const AttnParams& p);
 cudaError_t launch_flash_attention(const DeviceCtx& ctx, const AttnParams& p, cudaStream_t stream);
 
