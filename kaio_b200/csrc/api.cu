@@ -551,10 +551,10 @@ static int32_t run_int4(const kaio_f16* a, size_t a_len, const uint32_t* b, size
     pr.out = c;
     const __half* x = reinterpret_cast<const __half*>(a);
     if (w4a16_decode_ok(x, &pr, 1, m, n, k)) {
-        const size_t ws = w4a16_decode_workspace_bytes(*ctx, n, k);
-        if ((rc = ensure_workspace(ctx, s, ws, w4a16_decode_num_counters(n), &sc)))
+        const size_t ws = w4a16_decode_workspace_bytes(*ctx);
+        if ((rc = ensure_workspace(ctx, s, ws, w4a16_decode_num_counters(1, n), &sc)))
             return rc;
-        return finish(launch_w4a16_decode(*ctx, x, pr, out_f16, m, n, k, sc->workspace,
+        return finish(launch_w4a16_decode(*ctx, x, &pr, 1, out_f16, m, n, k, sc->workspace,
                                           sc->tile_counters, s),
                       "matmul_int4", "w4a16_decode_splitk");
     }
@@ -592,6 +592,14 @@ static int32_t run_qkv(int wfmt, const char* op, const __half* x, DqProblem prob
         return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     StreamScratch* sc = nullptr;
+    if (wfmt == WFMT_S4_PACKED && !post_scale && w4a16_decode_ok(x, probs, 3, m, n, k)) {
+        if ((rc = ensure_workspace(ctx, s, w4a16_decode_workspace_bytes(*ctx),
+                                   w4a16_decode_num_counters(3, n), &sc)))
+            return rc;
+        return finish(launch_w4a16_decode(*ctx, x, probs, 3, true, m, n, k, sc->workspace,
+                                          sc->tile_counters, s),
+                      op, "qkv_w4a16_decode_splitk");
+    }
     if (wfmt == WFMT_S4_PACKED && !post_scale && m <= fused_max_m() &&
         w4a16_fused_ok(x, probs, 3, m, n, k)) {
         const size_t ws = w4a16_fused_workspace_bytes(*ctx, 3, m, n, k);
@@ -1304,10 +1312,10 @@ static int32_t run_int4_allgather(const char* op, const kaio_f16* a, size_t a_le
     pr.out = copies.ptrs[rank];
     const __half* x = reinterpret_cast<const __half*>(a);
     if (w4a16_decode_ok(x, &pr, 1, m, n_loc, k)) {
-        if ((rc = ensure_workspace(ctx, s, w4a16_decode_workspace_bytes(*ctx, n_loc, k),
-                                   w4a16_decode_num_counters(n_loc), &sc)))
+        if ((rc = ensure_workspace(ctx, s, w4a16_decode_workspace_bytes(*ctx),
+                                   w4a16_decode_num_counters(1, n_loc), &sc)))
             return rc;
-        return finish(launch_w4a16_decode(*ctx, x, pr, true, m, n_loc, k, sc->workspace,
+        return finish(launch_w4a16_decode(*ctx, x, &pr, 1, true, m, n_loc, k, sc->workspace,
                                           sc->tile_counters, s, &copies),
                       op, "w4a16_decode_splitk_allgather");
     }
@@ -1464,10 +1472,10 @@ KAIO_API int32_t kaio_b200_matmul_int4_peer_partials(const kaio_f16* a, size_t a
     pr.out = copies.ptrs[rank];
     const __half* x = reinterpret_cast<const __half*>(a);
     if (w4a16_decode_ok(x, &pr, 1, m, n, k)) {
-        if ((rc = ensure_workspace(ctx, s, w4a16_decode_workspace_bytes(*ctx, n, k),
-                                   w4a16_decode_num_counters(n), &sc)))
+        if ((rc = ensure_workspace(ctx, s, w4a16_decode_workspace_bytes(*ctx),
+                                   w4a16_decode_num_counters(1, n), &sc)))
             return rc;
-        return finish(launch_w4a16_decode(*ctx, x, pr, false, m, n, k, sc->workspace,
+        return finish(launch_w4a16_decode(*ctx, x, &pr, 1, false, m, n, k, sc->workspace,
                                           sc->tile_counters, s, &copies),
                       op, "w4a16_decode_splitk_peer_partials");
     }
@@ -1585,7 +1593,7 @@ KAIO_API int32_t kaio_b200_allreduce_multimem_f32(const void* multicast_in, void
 // library holds these ~5.3 MB until the process exits).
 namespace kaio {
 constexpr size_t NOALLOC_MAX_CTAS = 320;         // two CTAs per SM; B200 has 148 SMs
-constexpr size_t NOALLOC_MAX_TILES = 4096;       // column tiles of 128 -> N <= 524288
+constexpr size_t NOALLOC_MAX_TILES = 16384;      // column tiles of 32 -> N <= 524288
 constexpr size_t NOALLOC_PARTIAL_BYTES = NOALLOC_MAX_CTAS * 2 * 16 * 128 * sizeof(float);
 constexpr size_t NOALLOC_COUNTER_BYTES = NOALLOC_MAX_TILES * sizeof(uint32_t);
 constexpr size_t NOALLOC_STATUS_BYTES = 256;
@@ -1620,10 +1628,10 @@ KAIO_API int32_t kaio_b200_matmul_int4_noalloc(const kaio_f16* a, size_t a_len,
         return fail(KAIO_B200_ERR_INVALID_CONFIG,
                     "%s: M must be at most 16 (got %u); larger M has no allocation-free variant",
                     op, m);
-    if (w4a16_decode_num_counters(n) > NOALLOC_MAX_TILES)
+    if (w4a16_decode_num_counters(1, n) > NOALLOC_MAX_TILES)
         return fail(KAIO_B200_ERR_INVALID_CONFIG,
                     "%s: N must be at most %zu (got %u): the fixed scratch holds %zu tile counters",
-                    op, NOALLOC_MAX_TILES * 128, n, NOALLOC_MAX_TILES);
+                    op, NOALLOC_MAX_TILES * 32, n, NOALLOC_MAX_TILES);
     DqProblem pr;
     pr.w = b_packed;
     pr.scales = reinterpret_cast<const __half*>(scales);
@@ -1671,10 +1679,10 @@ KAIO_API int32_t kaio_b200_matmul_int4_noalloc(const kaio_f16* a, size_t a_len,
     ctx.num_sms = g_noalloc_sms[dev];
     unsigned char* base = g_noalloc_ptr[dev];
     ctx.status = reinterpret_cast<uint32_t*>(base + NOALLOC_PARTIAL_BYTES + NOALLOC_COUNTER_BYTES);
-    if (w4a16_decode_workspace_bytes(ctx, n, k) > NOALLOC_PARTIAL_BYTES)
+    if (w4a16_decode_workspace_bytes(ctx) > NOALLOC_PARTIAL_BYTES)
         return fail(KAIO_B200_ERR_INVALID_CONFIG,
                     "%s: this device needs %zu bytes of split-K scratch, the fixed array holds %zu",
-                    op, w4a16_decode_workspace_bytes(ctx, n, k), NOALLOC_PARTIAL_BYTES);
+                    op, w4a16_decode_workspace_bytes(ctx), NOALLOC_PARTIAL_BYTES);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // The array keeps whatever the previous call left: the arrival counters must start at zero.
     // The status words are left alone, so that a wait that gave up in an earlier call stays
@@ -1682,7 +1690,7 @@ KAIO_API int32_t kaio_b200_matmul_int4_noalloc(const kaio_f16* a, size_t a_len,
     err = cudaMemsetAsync(base + NOALLOC_PARTIAL_BYTES, 0, NOALLOC_COUNTER_BYTES, s);
     if (err != cudaSuccess)
         return fail_cuda(err, "cudaMemsetAsync(noalloc scratch)");
-    return finish(launch_w4a16_decode(ctx, x, pr, false, m, n, k, base,
+    return finish(launch_w4a16_decode(ctx, x, &pr, 1, false, m, n, k, base,
                                       reinterpret_cast<uint32_t*>(base + NOALLOC_PARTIAL_BYTES), s),
                   op, "w4a16_decode_splitk_noalloc");
 }

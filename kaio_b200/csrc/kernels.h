@@ -76,12 +76,20 @@ cudaError_t launch_dq_generic(int wfmt, const __half* x, const DqProblem* probs,
 struct OutputCopies;
 bool w4a16_decode_ok(const void* x, const DqProblem* probs, int num_probs, uint32_t m, uint32_t n,
                      uint32_t k);
-size_t w4a16_decode_workspace_bytes(const DeviceCtx& ctx, uint32_t n, uint32_t k);
-size_t w4a16_decode_num_counters(uint32_t n);
-cudaError_t launch_w4a16_decode(const DeviceCtx& ctx, const __half* x, const DqProblem& prob,
-                                bool out_f16, uint32_t m, uint32_t n, uint32_t k, void* workspace,
-                                uint32_t* counters, cudaStream_t stream,
+size_t w4a16_decode_workspace_bytes(const DeviceCtx& ctx);
+size_t w4a16_decode_num_counters(int num_probs, uint32_t n);
+// One problem (with copies: stored to every destination) or three with the same n and x; picks
+// between the warp-level kernel and, for large matrices of 9 to 16 rows, the tcgen05 one.
+cudaError_t launch_w4a16_decode(const DeviceCtx& ctx, const __half* x, const DqProblem* probs,
+                                int num_probs, bool out_f16, uint32_t m, uint32_t n, uint32_t k,
+                                void* workspace, uint32_t* counters, cudaStream_t stream,
                                 const OutputCopies* copies = nullptr);
+
+size_t w4a16_decode_tc_workspace_bytes(const DeviceCtx& ctx);
+cudaError_t launch_w4a16_decode_tc(const DeviceCtx& ctx, const __half* x, const DqProblem& prob,
+                                   bool out_f16, uint32_t m, uint32_t n, uint32_t k, void* workspace,
+                                   uint32_t* counters, cudaStream_t stream,
+                                   const OutputCopies* copies);
 
 // Fused W4A16 GEMM for m > 16: int4 -> f16 dequantisation inside the GEMM (weights go from the
 // packed words to tensor memory, never to global memory as f16).  Needs no workspace.

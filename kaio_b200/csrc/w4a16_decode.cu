@@ -780,15 +780,6 @@ extern "C" __attribute__((visibility("default"))) int kaio_b200_debug_set_trace(
 }
 #endif
 
-bool w4a16_decode_ok(const void* x, const DqProblem* probs, int num_probs, uint32_t m, uint32_t n,
-                     uint32_t k)
-{
-    (void)n;
-    if (num_probs != 1 || m > 16 || k % 128 != 0)
-        return false;
-    return ((uintptr_t)x % 16 == 0) && ((uintptr_t)probs[0].w % 16 == 0);
-}
-
 static uint32_t decode_grid(const DeviceCtx& ctx, uint32_t n, uint32_t k)
 {
     const uint32_t units = ((n + w4dec::BN - 1) / w4dec::BN) * ((k + w4dec::BKK - 1) / w4dec::BKK);
@@ -796,19 +787,14 @@ static uint32_t decode_grid(const DeviceCtx& ctx, uint32_t n, uint32_t k)
     return units < ctas ? units : ctas;
 }
 
-size_t w4a16_decode_workspace_bytes(const DeviceCtx& ctx, uint32_t n, uint32_t k)
+size_t w4a16_decode_tc_workspace_bytes(const DeviceCtx& ctx)
 {
-    return (size_t)decode_grid(ctx, n, k) * 2 * w4dec::PARTIAL_FLOATS * sizeof(float);
+    return (size_t)ctx.num_sms * w4dec::CTAS_PER_SM * 2 * w4dec::PARTIAL_FLOATS * sizeof(float);
 }
 
-size_t w4a16_decode_num_counters(uint32_t n)
-{
-    return (n + w4dec::BN - 1) / w4dec::BN;
-}
-
-cudaError_t launch_w4a16_decode(const DeviceCtx& ctx, const __half* x, const DqProblem& prob,
-                                bool out_f16, uint32_t m, uint32_t n, uint32_t k, void* workspace,
-                                uint32_t* counters, cudaStream_t stream, const OutputCopies* copies)
+cudaError_t launch_w4a16_decode_tc(const DeviceCtx& ctx, const __half* x, const DqProblem& prob,
+                                   bool out_f16, uint32_t m, uint32_t n, uint32_t k, void* workspace,
+                                   uint32_t* counters, cudaStream_t stream, const OutputCopies* copies)
 {
     using namespace w4dec;
     CUtensorMap tmap_w;
