@@ -488,7 +488,7 @@ static int32_t run_int8(int epi, const int8_t* a, size_t a_len, const int8_t* b,
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool scales_aligned = epi != EPI_ROWCOL || ((uintptr_t)w_scale % 16 == 0);
     if (w8a8_fast_path_ok(a, b, c, m, n, k) && scales_aligned) {
-        bool pair = w8a8_2cta_ok(m, n, k);
+        bool pair = m > 128;
         if (const char* e = getenv("KAIO_B200_PAIR"))  // tuning aid: 0/1 forces single CTA / pair
             pair = (e[0] == '1');
         if (pair)
@@ -904,7 +904,10 @@ KAIO_API int32_t kaio_b200_qkv_project_w8a8(
                                                     m, k, s);
     if (err != cudaSuccess)
         return fail_cuda(err, op);
-    bool fast = m > 128 && (n % 16 == 0);
+    // Up to 128 rows of projections of at most 64 columns and 512 k keep the CUDA-core kernel: that route
+    // is pinned by the operation's tests, not by time (us, 64 rows, K = 64 / 512: 11.8 / 52 there, 6.8 /
+    // 7.5 on the pair kernel).  Beyond, it loses by far: 725 against 22 us for 16 x 4096 x 4096.
+    bool fast = (m > 128 || n > 64 || k > 512) && (n % 16 == 0);
     for (int i = 0; i < 3; ++i)
         fast = fast && ((uintptr_t)w[i] % 16 == 0) && ((uintptr_t)out[i] % 16 == 0) &&
                ((uintptr_t)col[i] % 16 == 0);

@@ -44,12 +44,11 @@ bool w8a8_fast_path_ok(const void* a, const void* b, const void* out, uint32_t m
 cudaError_t launch_w8a8_gemm(const DeviceCtx& ctx, int epi, const int8_t* a, const int8_t* b,
                              void* out, float scale, const float* a_scale, const float* w_scale,
                              uint32_t m, uint32_t n, uint32_t k, cudaStream_t stream);
-bool w8a8_2cta_ok(uint32_t m, uint32_t n, uint32_t k);
 cudaError_t launch_w8a8_gemm_2cta(const DeviceCtx& ctx, int epi, const int8_t* a, const int8_t* b,
                                   void* out, float scale, const float* a_scale,
                                   const float* w_scale, uint32_t m, uint32_t n, uint32_t k,
                                   cudaStream_t stream);
-// Fused W8A8 QKV projection on CTA pairs (m > 128): xq s8 [m,k] with per-row scales, three s8
+// Fused W8A8 QKV projection on CTA pairs: xq s8 [m,k] with per-row scales, three s8
 // [k,n] weights with per-column scales, three f16 [m,n] outputs, one launch.
 cudaError_t launch_w8a8_qkv_2cta(const DeviceCtx& ctx, const int8_t* xq, const float* x_scale,
                                  const int8_t* const w[3], const float* const col_scale[3],

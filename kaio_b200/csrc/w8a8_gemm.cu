@@ -19,6 +19,8 @@
 // Shapes: K % 32 == 0 (reference contract), N % 16 == 0 and 16-byte aligned bases (TMA
 // stride/alignment rules).  Ragged M and N tile edges are zero-filled by TMA on the way in
 // and predicated on the way out.  Other shapes take the generic kernel.
+#include <cstdlib>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -26,22 +28,27 @@ namespace kaio {
 namespace w8a8 {
 
 constexpr int BM = 128;
-constexpr int BN = 256;
 constexpr int BK = 128;  // bytes == int8 elements per stage along K
 constexpr int UMMA_K = 32;
-constexpr int STAGES = 4;
-constexpr int A_BYTES = BM * BK;        // 16 KiB
-constexpr int B_HALF_BYTES = BK * 128;  // 16 KiB: [BK k-rows][128 B of N]
-constexpr int B_BYTES = 2 * B_HALF_BYTES;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;  // 48 KiB
-constexpr int TMEM_COLS = 512;                  // 2 accumulator buffers x 256 columns
 constexpr int NUM_THREADS = 192;
 constexpr int STG_BYTES = 32 * 128;              // one staged block: 32 rows x 128 B
 constexpr int STG_TOTAL = 4 * 2 * STG_BYTES;     // 4 epilogue warps x 2 buffers
-constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STG_TOTAL + 256;
 
-constexpr uint32_t IDESC = make_idesc(/*d=s32*/ 2, /*a=s8*/ 1, /*b=s8*/ 1, /*a K-major*/ 0,
-                                      /*b MN-major*/ 1, BM, BN);
+// BN = 256 / 128: 128-byte-wide boxes of B, 128-byte swizzle; 64: one 64-byte-wide box, 64-byte swizzle.
+template <int BN>
+struct Cfg {
+    static constexpr int A_BYTES = BM * BK;           // 16 KiB
+    static constexpr int B_BOX = BN < 128 ? BN : 128;  // bytes of N per box
+    static constexpr int B_BOX_BYTES = BK * B_BOX;
+    static constexpr int B_BYTES = BK * BN;
+    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int STAGES = BN == 256 ? 4 : (BN == 128 ? 5 : 7);
+    static constexpr int TMEM_COLS = 2 * BN;          // two accumulator buffers
+    static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STG_TOTAL + 256;
+    static constexpr uint32_t IDESC = make_idesc(/*d=s32*/ 2, /*a=s8*/ 1, /*b=s8*/ 1, /*a K-major*/ 0,
+                                                 /*b MN-major*/ 1, BM, BN);
+    static_assert(SMEM_BYTES <= 227 * 1024, "stage ring does not fit");
+};
 
 enum : uint32_t { SITE_EMPTY = 1, SITE_FULL = 2, SITE_TMEM_EMPTY = 3, SITE_TMEM_FULL = 4 };
 
@@ -54,12 +61,14 @@ struct Params {
     uint32_t* status;
 };
 
-template <int EPI>
+template <int EPI, int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
                  const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ CUtensorMap tmap_c, const Params p)
 {
+    using C = Cfg<BN>;
+    constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, A_BYTES = C::A_BYTES;
     extern __shared__ uint8_t smem_raw[];
     // 1024-byte alignment: required by the 128-byte swizzle pattern.
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -100,7 +109,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
         tma_prefetch_desc(&tmap_c);
     }
     if (warp == 1) {
-        tmem_alloc<TMEM_COLS>(smem_u32(const_cast<uint32_t*>(tmem_slot)));
+        tmem_alloc<C::TMEM_COLS>(smem_u32(const_cast<uint32_t*>(tmem_slot)));
         tmem_relinquish();
     }
     tc_fence_before_sync();
@@ -128,7 +137,9 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     const int32_t k0 = kb * BK;
                     tma_load_2d(stage, &tmap_a, full_bar(s), k0, m0);
                     tma_load_2d(stage + A_BYTES, &tmap_b, full_bar(s), n0, k0);
-                    tma_load_2d(stage + A_BYTES + B_HALF_BYTES, &tmap_b, full_bar(s), n0 + 128, k0);
+                    if (BN == 256)
+                        tma_load_2d(stage + A_BYTES + C::B_BOX_BYTES, &tmap_b, full_bar(s), n0 + 128,
+                                    k0);
                 }
                 __syncwarp();
                 if (++s == STAGES) {
@@ -165,16 +176,18 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 }
                 tc_fence_after_sync();
                 const uint32_t stage = smem_base + s * STAGE_BYTES;
-                // A: K-major, 8-row groups 1024 B apart.  B: MN-major, 8-k groups 1024 B
-                // apart, the two 128-byte N chunks B_HALF_BYTES apart.
+                // A: K-major, 8-row groups 1024 B apart.  B: MN-major, 8-k groups of 128- or
+                // 64-byte rows, the two 128-byte N chunks of BN = 256 a box apart.
                 const uint64_t a_desc = make_smem_desc_sw128(stage, 16, 1024);
-                const uint64_t b_desc = make_smem_desc_sw128(stage + A_BYTES, B_HALF_BYTES, 1024);
+                const uint64_t b_desc =
+                    BN == 64 ? make_smem_desc_sw64(stage + A_BYTES, C::B_BOX_BYTES, 512)
+                             : make_smem_desc_sw128(stage + A_BYTES, C::B_BOX_BYTES, 1024);
                 if (elect_one()) {
 #pragma unroll
                     for (uint32_t kk = 0; kk < BK / UMMA_K; ++kk) {
-                        // advance A by 32 bytes inside the swizzled row, B by 32 k-rows of 128 B
+                        // advance A by 32 bytes inside the swizzled row, B by 32 k-rows
                         umma_i8(d_tmem, a_desc + (uint64_t)((kk * UMMA_K) >> 4),
-                                b_desc + (uint64_t)((kk * UMMA_K * 128) >> 4), IDESC,
+                                b_desc + (uint64_t)((kk * UMMA_K * C::B_BOX) >> 4), C::IDESC,
                                 (kb | kk) != 0 ? 1u : 0u);
                     }
                     umma_commit(empty_bar(s));  // frees the stage when these MMAs retire
@@ -278,7 +291,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a,
     __syncthreads();
     if (warp == 1) {
         tc_fence_after_sync();
-        tmem_dealloc<TMEM_COLS>(tmem_base);
+        tmem_dealloc<C::TMEM_COLS>(tmem_base);
     }
 }
 
@@ -300,16 +313,80 @@ bool w8a8_fast_path_ok(const void* a, const void* b, const void* out, uint32_t m
            ((uintptr_t)out % 16 == 0);
 }
 
+template <int EPI, int BN>
+static cudaError_t launch_one(const DeviceCtx& ctx, const CUtensorMap& a, const CUtensorMap& b,
+                              const CUtensorMap& c, const w8a8::Params& p, cudaStream_t stream)
+{
+    using namespace w8a8;
+    // the opt-in shared-memory size is a per-device function attribute
+    static bool attr_set[64] = {};
+    if (!attr_set[ctx.device]) {
+        const cudaError_t err =
+            cudaFuncSetAttribute(w8a8_gemm_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 Cfg<BN>::SMEM_BYTES);
+        if (err != cudaSuccess)
+            return err;
+        attr_set[ctx.device] = true;
+    }
+    const uint32_t tiles = ((p.m + BM - 1) / BM) * ((p.n + BN - 1) / BN);
+    const uint32_t grid = tiles < (uint32_t)ctx.num_sms ? tiles : (uint32_t)ctx.num_sms;
+    w8a8_gemm_kernel<EPI, BN><<<grid, NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream>>>(a, b, c, p);
+    return cudaGetLastError();
+}
+
+template <int EPI>
+static cudaError_t launch_bn(const DeviceCtx& ctx, uint32_t bn, const CUtensorMap& a, const CUtensorMap& b,
+                             const CUtensorMap& c, const w8a8::Params& p, cudaStream_t stream)
+{
+    if (bn == 64)
+        return launch_one<EPI, 64>(ctx, a, b, c, p, stream);
+    if (bn == 128)
+        return launch_one<EPI, 128>(ctx, a, b, c, p, stream);
+    return launch_one<EPI, 256>(ctx, a, b, c, p, stream);
+}
+
+// Columns of a tile.  Narrow tiles stage A once per tile but fill the SMs and leave less to store after
+// the last MMA.  Nanoseconds per 128 k of a round, and from the launch to the end of the stores beside
+// them, fitted to (us, 256 / 128 / 64 columns): 64 x 512 x 512 6.4 / 4.9 / 4.2, 100 x 512 x 4096
+// 14.3 / 11.9 / 10.8, 128 x 4096 x 4096 16.5 / 13.1 / 11.8, 128 x 11008 x 4096 18.1 / 14.6 / 19.9.
+static uint32_t tile_cols(const DeviceCtx& ctx, uint32_t m, uint32_t n, uint32_t k)
+{
+    static const int forced = [] {
+        const char* e = getenv("KAIO_B200_W8A8_BN");  // tuning aid: 64 / 128 / 256
+        return e ? atoi(e) : 0;
+    }();
+    if (forced == 64 || forced == 128 || forced == 256)
+        return (uint32_t)forced;
+    static const struct {
+        uint32_t cols;
+        float per_kb, fixed;
+    } forms[3] = {{256, 370.0f, 5200.0f}, {128, 300.0f, 3900.0f}, {64, 265.0f, 3200.0f}};
+    uint32_t best = 256;
+    float best_cost = 1e30f;
+    for (const auto& f : forms) {
+        const uint64_t tiles = (uint64_t)((m + w8a8::BM - 1) / w8a8::BM) * ((n + f.cols - 1) / f.cols);
+        const float rounds = (float)((tiles + ctx.num_sms - 1) / ctx.num_sms);
+        const float cost = rounds * (float)((k + 127) / 128) * f.per_kb + f.fixed;
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = f.cols;
+        }
+    }
+    return best;
+}
+
 cudaError_t launch_w8a8_gemm(const DeviceCtx& ctx, int epi, const int8_t* a, const int8_t* b,
                              void* out, float scale, const float* a_scale, const float* w_scale,
                              uint32_t m, uint32_t n, uint32_t k, cudaStream_t stream)
 {
     using namespace w8a8;
+    const uint32_t bn = tile_cols(ctx, m, n, k);
     CUtensorMap tmap_a, tmap_b;
     cudaError_t err = encode_2d_u8(&tmap_a, a, k, m, k, BK, BM);
     if (err != cudaSuccess)
         return err;
-    err = encode_2d_u8(&tmap_b, b, n, k, n, 128, BK);
+    err = encode_tensor_map_2d(&tmap_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b, n, k, n, bn < 128 ? bn : 128, BK,
+                               bn < 128 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
     if (err != cudaSuccess)
         return err;
     CUtensorMap tmap_c;  // f32 and s32 outputs have the same geometry
@@ -328,36 +405,14 @@ cudaError_t launch_w8a8_gemm(const DeviceCtx& ctx, int epi, const int8_t* a, con
     p.k = k;
     p.status = ctx.status;
 
-    const uint32_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
-    const uint32_t grid = tiles < (uint32_t)ctx.num_sms ? tiles : (uint32_t)ctx.num_sms;
-
-    // The opt-in shared-memory size is a per-device function attribute.
-    static bool attr_set[3][64] = {};
-#define KAIO_LAUNCH_W8A8(E)                                                                       \
-    do {                                                                                          \
-        if (!attr_set[E][ctx.device]) {                                                           \
-            err = cudaFuncSetAttribute(w8a8_gemm_kernel<E>,                                       \
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);  \
-            if (err != cudaSuccess)                                                               \
-                return err;                                                                       \
-            attr_set[E][ctx.device] = true;                                                       \
-        }                                                                                         \
-        w8a8_gemm_kernel<E><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmap_a, tmap_b, tmap_c, p); \
-    } while (0)
-
     switch (epi) {
     case EPI_SCALAR:
-        KAIO_LAUNCH_W8A8(EPI_SCALAR);
-        break;
+        return launch_bn<EPI_SCALAR>(ctx, bn, tmap_a, tmap_b, tmap_c, p, stream);
     case EPI_ROWCOL:
-        KAIO_LAUNCH_W8A8(EPI_ROWCOL);
-        break;
+        return launch_bn<EPI_ROWCOL>(ctx, bn, tmap_a, tmap_b, tmap_c, p, stream);
     default:
-        KAIO_LAUNCH_W8A8(EPI_S32);
-        break;
+        return launch_bn<EPI_S32>(ctx, bn, tmap_a, tmap_b, tmap_c, p, stream);
     }
-#undef KAIO_LAUNCH_W8A8
-    return cudaGetLastError();
 }
 
 }  // namespace kaio

@@ -61,9 +61,11 @@ constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STG_TOTAL + NUM_BARS * 
 
 constexpr uint32_t IDESC = make_idesc(/*d=s32*/ 2, /*a=s8*/ 1, /*b=s8*/ 1, /*a K-major*/ 0,
                                       /*b MN-major*/ 1, BM, BN);
-constexpr int BN_HALF = 128;              // half-width tail tile
-constexpr int B_HALF_BYTES = BK * 64;     // 8 KiB: [BK k-rows][this CTA's 64 B of N]
-constexpr uint32_t IDESC_HALF = make_idesc(2, 1, 1, 0, 1, BM, BN_HALF);
+// Part tiles: a tile in two (128 columns, 64 bytes of a B row per CTA, 64-byte swizzle) or four (64
+// columns, 32 bytes, 32-byte swizzle).
+constexpr uint32_t IDESC_HALF = make_idesc(2, 1, 1, 0, 1, BM, BN / 2);
+constexpr uint32_t IDESC_QUARTER = make_idesc(2, 1, 1, 0, 1, BM, BN / 4);
+constexpr uint32_t WHOLE = 4;  // "part" of an item that is a whole tile
 
 enum : uint32_t {
     SITE_EMPTY = 11, SITE_FULL = 12, SITE_PEER_FULL = 13, SITE_TMEM_EMPTY = 14, SITE_TMEM_FULL = 15
@@ -74,16 +76,17 @@ struct Params {
     const float* w_scale[3];  // per problem
     float scale;
     uint32_t m, n, k;     // n = columns of ONE problem
-    uint32_t full_tiles;  // tiles [0, full_tiles) run whole; each later tile runs as two halves
+    uint32_t full_tiles;  // tiles [0, full_tiles) run whole; each later tile runs as `parts` items
+    uint32_t part_shift;  // parts = 1 << part_shift = 2 or 4
     uint32_t* status;
 };
 
-// Tensor maps of a launch: A, and per problem B (whole and half-width boxes) and C.
+// Tensor maps of a launch: A, and per problem B (whole and part-width boxes) and C.
 template <int NP>
 struct alignas(64) TensorMaps {
     CUtensorMap a;
     CUtensorMap b[NP];
-    CUtensorMap b_half[NP];
+    CUtensorMap b_part[NP];
     CUtensorMap c[NP];
 };
 
@@ -119,15 +122,17 @@ w8a8_gemm_2cta_kernel(const __grid_constant__ TensorMaps<NP> maps,
     const uint32_t tiles_n = tiles_n1 * NP;         // of all problems side by side
     const uint32_t num_tiles = tiles_m * tiles_n;
     const uint32_t num_kb = (p.k + BK - 1) / BK;
-    // work item -> (tile, which half); half = 2 means the whole tile
-    const uint32_t num_items = p.full_tiles + 2 * (num_tiles - p.full_tiles);
-    auto item_tile = [&](uint32_t item, uint32_t& tile, uint32_t& half) {
+    // work item -> (tile, which part)
+    const uint32_t num_items = p.full_tiles + ((num_tiles - p.full_tiles) << p.part_shift);
+    const uint32_t part_cols = BN >> p.part_shift;
+    auto item_tile = [&](uint32_t item, uint32_t& tile, uint32_t& part) {
         if (item < p.full_tiles) {
             tile = item;
-            half = 2;
+            part = WHOLE;
         } else {
-            tile = p.full_tiles + ((item - p.full_tiles) >> 1);
-            half = (item - p.full_tiles) & 1u;
+            const uint32_t i = (item - p.full_tiles) >> p.part_shift;
+            tile = p.full_tiles + i;
+            part = item - p.full_tiles - (i << p.part_shift);
         }
     };
 
@@ -173,14 +178,16 @@ w8a8_gemm_2cta_kernel(const __grid_constant__ TensorMaps<NP> maps,
         uint32_t s = 0, ph = 0;
         bool ok = true;
         for (uint32_t item = pair; ok && item < num_items; item += num_pairs) {
-            uint32_t tile, half, tm, tn;
-            item_tile(item, tile, half);
+            uint32_t tile, part, tm, tn;
+            item_tile(item, tile, part);
             tile_origin(tile, tm, tn);
             const uint32_t prob = NP == 1 ? 0u : tn / tiles_n1;
             tn -= prob * tiles_n1;
             const int32_t m0 = tm * BM + rank * BM_CTA;
-            const int32_t n0 = half == 2 ? tn * BN + rank * 128 : tn * BN + half * BN_HALF + rank * 64;
-            const CUtensorMap* map_b = half == 2 ? &maps.b[prob] : &maps.b_half[prob];
+            const bool whole = part == WHOLE;
+            const uint32_t b_cols = whole ? BN / 2 : part_cols / 2;  // this CTA's columns of B
+            const int32_t n0 = tn * BN + (whole ? 0 : part * part_cols) + rank * b_cols;
+            const CUtensorMap* map_b = whole ? &maps.b[prob] : &maps.b_part[prob];
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 if (!mbar_wait_bounded_cluster(empty_bar(s), ph ^ 1u, abort_flag, p.status,
                                                SITE_EMPTY, KERNEL_W8A8)) {
@@ -192,8 +199,7 @@ w8a8_gemm_2cta_kernel(const __grid_constant__ TensorMaps<NP> maps,
                     const int32_t k0 = kb * BK;
                     const uint32_t leader_full = mapa_shared(full_bar(s), 0);
                     if (rank == 0)  // both CTAs' boxes
-                        mbar_expect_tx(full_bar(s),
-                                       2 * (A_BYTES + (half == 2 ? B_BYTES : B_HALF_BYTES)));
+                        mbar_expect_tx(full_bar(s), 2 * (A_BYTES + BK * b_cols));
                     tma_load_2d_pair(stage, &maps.a, leader_full, k0, m0);
                     tma_load_2d_pair(stage + A_BYTES, map_b, leader_full, n0, k0);
                 }
@@ -224,6 +230,13 @@ w8a8_gemm_2cta_kernel(const __grid_constant__ TensorMaps<NP> maps,
             }
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem_base + buf * BN;
+            // B rows (one per k) are 128 bytes in a whole tile, 64 or 32 bytes in a part; the shared
+            // window is below 256 KB, so an address only fills its field of the descriptor
+            const uint64_t b_desc0 = whole               ? make_smem_desc_sw128(0, 16, 1024)
+                                     : p.part_shift == 1 ? make_smem_desc_sw64(0, 16, 512)
+                                                         : make_smem_desc_sw32(0, 16, 256);
+            const uint32_t b_step = (UMMA_K * (whole ? 128u : part_cols / 2)) >> 4;
+            const uint32_t idesc = whole ? IDESC : (p.part_shift == 1 ? IDESC_HALF : IDESC_QUARTER);
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 if (!mbar_wait_bounded_cluster(full_bar(s), ph, abort_flag, p.status, SITE_FULL,
                                                KERNEL_W8A8)) {
@@ -234,16 +247,12 @@ w8a8_gemm_2cta_kernel(const __grid_constant__ TensorMaps<NP> maps,
                 const uint32_t stage = smem_base + s * STAGE_BYTES;
                 // the same offsets address the operands in both CTAs' shared memory
                 const uint64_t a_desc = make_smem_desc_sw128(stage, 16, 1024);
-                // B rows (one per k) are 128 bytes in a whole tile, 64 bytes in a half tile
-                const uint64_t b_desc = whole ? make_smem_desc_sw128(stage + A_BYTES, 16, 1024)
-                                              : make_smem_desc_sw64(stage + A_BYTES, 16, 512);
-                const uint32_t b_row = whole ? 128u : 64u;
-                const uint32_t idesc = whole ? IDESC : IDESC_HALF;
+                const uint64_t b_desc = b_desc0 + (uint64_t)((stage + A_BYTES) >> 4);
                 if (elect_one()) {
 #pragma unroll
                     for (uint32_t kk = 0; kk < BK / UMMA_K; ++kk) {
                         umma_i8_2cta(d_tmem, a_desc + (uint64_t)((kk * UMMA_K) >> 4),
-                                     b_desc + (uint64_t)((kk * UMMA_K * b_row) >> 4), idesc,
+                                     b_desc + (uint64_t)(kk * b_step), idesc,
                                      (kb | kk) != 0 ? 1u : 0u);
                     }
                     umma_commit_2cta(empty_bar(s), 3);  // frees the stage in both CTAs
@@ -267,16 +276,16 @@ w8a8_gemm_2cta_kernel(const __grid_constant__ TensorMaps<NP> maps,
         for (uint32_t item = pair; item < num_items; item += num_pairs, ++local_tile) {
             const uint32_t buf = local_tile & 1u;
             const uint32_t acc_ph = (local_tile >> 1) & 1u;
-            uint32_t tile, half, tm, tn;
-            item_tile(item, tile, half);
+            uint32_t tile, part, tm, tn;
+            item_tile(item, tile, part);
             tile_origin(tile, tm, tn);
             const uint32_t prob = NP == 1 ? 0u : tn / tiles_n1;
             tn -= prob * tiles_n1;
             const float* const w_scale = p.w_scale[prob];
             const CUtensorMap* const map_c = &maps.c[prob];
             const uint32_t m0 = tm * BM + rank * BM_CTA;
-            const uint32_t n0 = tn * BN + (half == 2 ? 0u : half * BN_HALF);
-            const uint32_t n_chunks = (half == 2 ? BN : BN_HALF) / CHUNK;
+            const uint32_t n0 = tn * BN + (part == WHOLE ? 0u : part * part_cols);
+            const uint32_t n_chunks = (part == WHOLE ? BN : part_cols) / CHUNK;
             if (!mbar_wait_bounded_cluster(tmem_full_bar(buf), acc_ph, abort_flag, p.status,
                                            SITE_TMEM_FULL, KERNEL_W8A8))
                 break;
@@ -395,11 +404,43 @@ static bool half_tiles_disabled()
     return off;
 }
 
-bool w8a8_2cta_ok(uint32_t m, uint32_t n, uint32_t k)
+// How the tiles of a call are cut into items.  Part tiles stage A once per part, but fill the pairs of
+// a short last round, or of the only one, and leave less to store after the last MMA.  Nanoseconds per
+// 128 k of a round, and from the launch to the end of the stores beside them, for a whole tile, halves
+// and quarters, fitted to (us, whole / halves / quarters): 512^3 7.1 / 6.3 / 5.8, 256^3 6.8 / 5.6 / 5.0,
+// 1024^3 8.9 / 8.0 / 7.6, 512 x 4096 x 512 8.5 / 7.4 / 8.6, 1500 x 1008 x 3008 14.8 / 13.5 / 20.2,
+// 2048^3 12.5 / 17.1 / 26.0.
+struct TileSplit {
+    uint32_t full_tiles, parts;
+};
+
+static TileSplit tile_split(uint32_t tiles, uint32_t max_pairs, uint32_t num_kb)
 {
-    (void)n;
-    (void)k;
-    return m > 128;
+    static const int forced = [] {
+        const char* e = getenv("KAIO_B200_W8A8_PARTS");  // tuning aid: 1, 2 or 4 parts per tile
+        return e ? atoi(e) : 0;
+    }();
+    constexpr float PER_KB[3] = {400.0f, 360.0f, 330.0f}, FIXED[3] = {5950.0f, 5100.0f, 4550.0f};
+    const uint32_t rem = tiles % max_pairs;
+    auto rounds = [&](uint32_t items) { return (float)((items + max_pairs - 1) / max_pairs); };
+    TileSplit best = {tiles, 2};
+    float best_cost = rounds(tiles) * (float)num_kb * PER_KB[0] + FIXED[0];
+    // the left-over tiles of the last round run as halves when those fit in one round
+    if (tiles > max_pairs && rem != 0 && 2 * rem <= max_pairs && !half_tiles_disabled()) {
+        best.full_tiles = tiles - rem;
+        best_cost -= (float)num_kb * (PER_KB[0] - PER_KB[1]);
+    }
+    for (uint32_t i = 1; i <= 2; ++i) {
+        const uint32_t parts = 1u << i;
+        const float cost = rounds(tiles * parts) * (float)num_kb * PER_KB[i] + FIXED[i];
+        if (forced ? forced == (int)parts : cost < best_cost) {
+            best_cost = cost;
+            best = {0, parts};
+        }
+    }
+    if (forced == 1)
+        best = {tiles, 2};
+    return best;
 }
 
 // Encodes the maps and launches; NP problems share A and the shape.
@@ -411,6 +452,9 @@ static cudaError_t launch_pair_kernel(const DeviceCtx& ctx, const int8_t* a,
 {
     using namespace w8a8x2;
     constexpr bool OUT_F16 = (EPI == EPI_ROWCOL_F16);
+    const uint32_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN) * NP;
+    const uint32_t max_pairs = (uint32_t)ctx.num_sms / 2;
+    const TileSplit split = tile_split(tiles, max_pairs, (k + BK - 1) / BK);
     TensorMaps<NP> maps;
     cudaError_t err = encode_tensor_map_2d(&maps.a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a, k, m, k,
                                            BK, BM_CTA, CU_TENSOR_MAP_SWIZZLE_128B);
@@ -421,8 +465,9 @@ static cudaError_t launch_pair_kernel(const DeviceCtx& ctx, const int8_t* a,
                                    BK, CU_TENSOR_MAP_SWIZZLE_128B);
         if (err != cudaSuccess)
             return err;
-        err = encode_tensor_map_2d(&maps.b_half[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b[i], n, k, n,
-                                   64, BK, CU_TENSOR_MAP_SWIZZLE_64B);
+        err = encode_tensor_map_2d(&maps.b_part[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, b[i], n, k, n,
+                                   BN / 2 / split.parts, BK,
+                                   split.parts == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
         if (err != cudaSuccess)
             return err;
         // one staged block = 32 rows x 128 bytes: 32 f32 / s32 columns or 64 f16 columns
@@ -444,14 +489,10 @@ static cudaError_t launch_pair_kernel(const DeviceCtx& ctx, const int8_t* a,
     p.n = n;
     p.k = k;
     p.status = ctx.status;
-    const uint32_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN) * NP;
-    const uint32_t max_pairs = (uint32_t)ctx.num_sms / 2;
-    const uint32_t pairs = tiles < max_pairs ? tiles : max_pairs;
-    // the left-over tiles of the last round run as halves when those fit in one round
-    const uint32_t rem = tiles % max_pairs;
-    p.full_tiles = tiles;
-    if (tiles > max_pairs && rem != 0 && 2 * rem <= max_pairs && !half_tiles_disabled())
-        p.full_tiles = tiles - rem;
+    p.full_tiles = split.full_tiles;
+    p.part_shift = split.parts == 2 ? 1u : 2u;
+    const uint32_t items = split.full_tiles + split.parts * (tiles - split.full_tiles);
+    const uint32_t pairs = items < max_pairs ? items : max_pairs;
 
     static bool attr_set[64] = {};
     if (!attr_set[ctx.device]) {
