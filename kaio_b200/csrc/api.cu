@@ -514,14 +514,15 @@ static uint32_t fused_max_m()
     return v;
 }
 
-// Largest M the fused W8A16 kernel takes: up to 256 rows one tile holds them all and every weight is
-// converted once.  KAIO_B200_W8A16_FUSED_MAX_M overrides it (tuning aid).
+// Largest M the fused W8A16 kernel takes: two 256-row tiles, every weight converted at most twice.  us,
+// two launches / this kernel, three 4096 x 4096 projections: M = 300 92 / 60, M = 512 93 / 66.
+// KAIO_B200_W8A16_FUSED_MAX_M overrides it (tuning aid).
 static uint32_t w8a16_fused_max_m()
 {
     static const uint32_t v = [] {
         if (const char* e = getenv("KAIO_B200_W8A16_FUSED_MAX_M"))
             return (uint32_t)strtoul(e, nullptr, 10);
-        return 256u;
+        return 512u;
     }();
     return v;
 }

@@ -13,11 +13,10 @@
 //  * the weights go [64 k][128 columns] s8 by TMA -> f16 in the 128-byte swizzle that tcgen05 reads
 //    MN-major (columns are contiguous in both, so the conversion never transposes) and the
 //    activations by TMA as the K-major operand;
-//  * the K range of a tile is cut over the CTAs of a cluster until there is about a CTA and a half
-//    per SM; the partial tiles meet in distributed shared memory, in rank order: no scratch, no
-//    atomics, one launch.
-// Measured (three projections, weights from HBM): 2048 x 2048, M = 64: 38.9 -> 17.2 us; 4096 x 4096,
-// M = 16 / 128 / 256: 24 / 34 / 46 us.
+//  * the K range of a tile is cut over the CTAs of a cluster while they all run at once; the partial
+//    tiles meet in distributed shared memory, in rank order: no scratch, no atomics, one launch.
+// Measured (us, three projections, weights from HBM, two launches -> this one): 2048 x 2048, M = 64:
+// 38.9 -> 12.1; 4096 x 4096, M = 300 / 512: 92 / 93 -> 60 / 66; M = 16 / 128 / 256: 23 / 30 / 36.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -376,12 +375,18 @@ cudaError_t launch_w8a16_fused(const DeviceCtx& ctx, const __half* x, const DqPr
     p.tiles_n = (n + BN - 1) / BN;
     p.status = ctx.status;
     const uint32_t tiles = p.tiles_n * (uint32_t)num_probs, tiles_m = (m + nrows - 1) / nrows;
-    // K is cut until there are three CTAs for every two SMs (two of them fit an SM up to 128 rows; the
-    // 256-row form has one), each with four K blocks at least to cover the fill of its pipeline.
-    const uint32_t want = nrows <= 128 ? ctx.num_sms * 3 / 2 : ctx.num_sms * 3 / 4;
+    // K is cut as long as all CTAs run at once (two fit an SM up to 128 rows, the 256-row form has one)
+    // and keep eight K blocks each to cover the fill of their pipeline and the sum over the cluster.  us
+    // for a cut in 1 / 2 / 4 / 8: 2048 x 2048, M = 64 17.3 / 12.7 / 12.1 / 17.3 (48 tiles); K x N = 4096 x
+    // 4096, M = 16 27.9 / 23.2 / 24.1 / 30.0 (96 tiles), M = 256 35.9 / 46 / 49 / 89; 8192 x 1024, M = 16
+    // 51 / 29 / 17 / 15 (24 tiles).  With more tiles than SMs a long K is still cut once, for the balance:
+    // 8192 x 8192, M = 8 74 / 65 / 67 / 82 (192 tiles).
+    const uint32_t ctas = tiles * tiles_m, slots = nrows <= 128 ? 2 * ctx.num_sms : ctx.num_sms;
     uint32_t split = 1;
-    while (split < MAX_SPLIT && tiles * tiles_m * split < want && p.num_kb >= 8 * split)
+    while (split < MAX_SPLIT && ctas * split * 2 <= slots && p.num_kb >= 16 * split)
         split *= 2;
+    if (nrows <= 128 && split == 1 && ctas > (uint32_t)ctx.num_sms && ctas <= slots && p.num_kb >= 128)
+        split = 2;
     switch (nrows) {
     case 32:
         return launch<32>(maps, p, tiles, tiles_m, split, ctx.device, stream);

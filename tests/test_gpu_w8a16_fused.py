@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("col", [False, True])
 @pytest.mark.parametrize("m,n,k", [(1, 16, 16), (32, 144, 80), (33, 128, 1024), (64, 1040, 2048), (65, 256, 528),
-                                   (128, 272, 4096), (129, 128, 640), (256, 400, 1008)])
+                                   (128, 272, 4096), (129, 128, 640), (256, 400, 1008),
+                                   (257, 144, 512), (512, 128, 2048)])
 def test_fused(oracle, m, n, k, col):
     rng = np.random.default_rng(m + n + k)
     x = rng.standard_normal(m * k).astype(np.float16)
