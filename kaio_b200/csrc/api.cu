@@ -226,6 +226,10 @@ static int32_t ensure_workspace(DeviceCtx* c, cudaStream_t stream, size_t bytes,
     *out = sc;
     if (bytes <= sc->workspace_bytes && counters <= sc->num_tile_counters)
         return KAIO_B200_OK;
+    // 64 KB of counters from the start (the kernels' column tiles differ, a call of one should not
+    // make the next one of another grow them)
+    if (counters > sc->num_tile_counters && counters < 16384)
+        counters = 16384;
     int32_t rc = refuse_growth_in_capture(stream, "split-K scratch");
     if (rc)
         return rc;
@@ -254,6 +258,22 @@ static int32_t ensure_workspace(DeviceCtx* c, cudaStream_t stream, size_t bytes,
         sc->num_tile_counters = counters;
     }
     return KAIO_B200_OK;
+}
+
+// A fused QKV call of many rows leaves the split-K scratch of the same projections' decode step behind,
+// so that warming the op at its largest shape still covers a decode step captured later.  Not during a
+// capture, and a failure is the later call's to report.
+static void prepare_decode_scratch(DeviceCtx* c, cudaStream_t stream, int num_probs, uint32_t n)
+{
+    StreamScratch* sc = scratch_for(c, stream);
+    const size_t bytes = w4a16_decode_workspace_bytes(*c), counters = w4a16_decode_num_counters(num_probs, n);
+    if (bytes <= sc->workspace_bytes && counters <= sc->num_tile_counters)
+        return;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone)
+        return;
+    if (ensure_workspace(c, stream, bytes, counters, &sc) != KAIO_B200_OK)
+        cudaGetLastError();
 }
 
 // The dequantised-weight workspace is written and read by the dequantising GEMM calls of one
@@ -614,6 +634,8 @@ static int32_t run_qkv(int wfmt, const char* op, const __half* x, DqProblem prob
     if (wfmt == WFMT_S8_ROWMAJOR && post_scale && m <= w8a16_fused_max_m() &&
         w8a16_fused_ok(x, probs, 3, m, n, k))
         return finish(launch_w8a16_fused(*ctx, x, probs, 3, m, n, k, s), op, "qkv_w8a16_fused");
+    if (wfmt == WFMT_S4_PACKED && w4a16_decode_ok(x, probs, 3, 1, n, k))
+        prepare_decode_scratch(ctx, s, 3, n);
     if (dq_gemm_fast_path_ok(wfmt, x, probs, 3, true, m, n, k)) {
         if ((rc = ensure_dq_workspace(ctx, s, dq_gemm_workspace_bytes(3, n, k), &sc)))
             return rc;

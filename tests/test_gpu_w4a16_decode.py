@@ -43,3 +43,27 @@ def test_qkv(oracle, m, n, k):
     assert ops.last_variant() == "qkv_w4a16_decode_splitk"
     for got, (w, s) in zip(o, ws):
         assert max_rel(host(got, (m, n)), oracle.qkv_int4(x, w, s, m, n, k)) < 1e-3
+
+
+def test_qkv_decode_capture_after_warming_many_rows(oracle):
+    """Warming the op at its largest shape covers a decode step captured later on that stream."""
+    n, k, m = 256, 512, 4
+    rng = np.random.default_rng(3)
+    ws = [weights(oracle, rng, k, n) for _ in range(3)]
+    wd, sd = [dev(w) for w, _ in ws], [dev(s) for _, s in ws]
+    x = rng.standard_normal(600 * k).astype(np.float16)
+    xd = dev(x)
+    o = [torch.zeros((600 * n,), device="cuda", dtype=torch.float16) for _ in range(3)]
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        ops.qkv_project_int4(device(), xd, *wd, *sd, *o, 600, n, k, G)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            ops.qkv_project_int4(device(), xd, *wd, *sd, *o, m, n, k, G)
+        for t in o:
+            t.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+    for got, (w, s) in zip(o, ws):
+        assert max_rel(host(got)[:m * n].reshape(m, n), oracle.qkv_int4(x[:m * k], w, s, m, n, k)) < 1e-3
