@@ -223,15 +223,20 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
         : "memory");
 }
 
-// First unit of CTA c when `units` units are cut into `grid` contiguous ranges.
+// First unit of CTA c when `units` units are cut into `grid` contiguous ranges: c * units / grid in
+// 32-bit steps (grid^2 is below 2^32).  As 64-bit quotients the ranges cost 1 to 2 us of a launch of 15 to 42: they stand
+// in front of the first load and in the chain behind the last product.
 __device__ __forceinline__ uint32_t range_begin(uint32_t c, uint32_t units, uint32_t grid)
 {
-    return (uint32_t)(((uint64_t)c * units) / grid);
+    const uint32_t len = units / grid, rem = units - len * grid;
+    return c * len + c * rem / grid;
 }
 
 // The CTA whose range holds unit u.
 __device__ __forceinline__ uint32_t owner_of(uint32_t u, uint32_t units, uint32_t grid)
 {
+    if (__umulhi(units, grid) == 0)  // (u + 1) * grid fits 32 bits
+        return ((u + 1) * grid - 1) / units;
     return (uint32_t)((((uint64_t)u + 1) * grid - 1) / units);
 }
 
@@ -712,8 +717,9 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmap_w,
                         acc[i] = 0.0f;
 #pragma unroll 2  // two contributors' loads in flight
                     for (uint32_t c = c_first; c <= c_last; ++c) {
-                        const uint32_t c_tile0 = range_begin(c, units, gridDim.x) / p.num_kb;
-                        const uint32_t cslot = (tile == c_tile0) ? 0u : 1u;
+                        // the tile opens c's range unless an earlier one does
+                        const uint32_t cslot =
+                            range_begin(c, units, gridDim.x) >= tile * p.num_kb ? 0u : 1u;
                         const float* src =
                             p.partials + ((size_t)(c * 2 + cslot) * PARTIAL_FLOATS) + tid * 16;
 #pragma unroll

@@ -122,15 +122,20 @@ __device__ __forceinline__ void fence_acq_rel_gpu()
     asm volatile("fence.acq_rel.gpu;" ::: "memory");
 }
 
-// First unit of CTA c when `units` units are cut into `grid` contiguous ranges.
+// First unit of CTA c when `units` units are cut into `grid` contiguous ranges: c * units / grid in
+// 32-bit steps (grid^2 is below 2^32).  As 64-bit quotients the ranges cost 4 us of a launch of 27: they stand
+// in front of the first load and in the chain behind the last product.
 __device__ __forceinline__ uint32_t range_begin(uint32_t c, uint32_t units, uint32_t grid)
 {
-    return (uint32_t)(((uint64_t)c * units) / grid);
+    const uint32_t len = units / grid, rem = units - len * grid;
+    return c * len + c * rem / grid;
 }
 
 // The CTA whose range holds unit u.
 __device__ __forceinline__ uint32_t owner_of(uint32_t u, uint32_t units, uint32_t grid)
 {
+    if (__umulhi(units, grid) == 0)  // (u + 1) * grid fits 32 bits
+        return ((u + 1) * grid - 1) / units;
     return (uint32_t)((((uint64_t)u + 1) * grid - 1) / units);
 }
 
@@ -577,8 +582,9 @@ w4a16_fused_kernel(const __grid_constant__ TensorMaps maps, const Params p)
                     acc[i] = 0.0f;
 #pragma unroll 2  // two contributors' loads in flight
                 for (uint32_t cc = c_first; cc <= c_last; ++cc) {  // ascending: a fixed order
-                    const uint32_t cc_tile0 = range_begin(cc, units, gridDim.x) / num_kb;
-                    const uint32_t cslot = (g.tile == cc_tile0) ? 0u : 1u;
+                    // the tile opens cc's range unless an earlier one does
+                    const uint32_t cslot =
+                        range_begin(cc, units, gridDim.x) >= g.tile * num_kb ? 0u : 1u;
                     const float4* src = p.partials + (size_t)(cc * 2 + cslot) * PART_F4 + tid;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
