@@ -123,7 +123,7 @@ __device__ __forceinline__ void fence_acq_rel_gpu()
 }
 
 // First unit of CTA c when `units` units are cut into `grid` contiguous ranges: c * units / grid in
-// 32-bit steps (grid^2 is below 2^32).  As 64-bit quotients the ranges cost 4 us of a launch of 27: they stand
+// 32-bit steps (grid^2 is below 2^32).  As 64-bit quotients the ranges cost 2 us of the 154 of 28672 x 8192 at M = 250: they stand
 // in front of the first load and in the chain behind the last product.
 __device__ __forceinline__ uint32_t range_begin(uint32_t c, uint32_t units, uint32_t grid)
 {
