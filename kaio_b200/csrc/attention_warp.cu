@@ -10,7 +10,9 @@
 // results are merged in shared memory.  Long, head_dim 64: the tensor pipe and the exponentials, four
 // warps of 16 rows over common 64-key stages, two in flight.
 // Precision: P enters the second product as hi + lo, two f16 numbers that hold 22 bits of it (scaled
-// by 2^12 so that lo stays clear of f16's subnormals), because the scalar kernel kept it in f32.
+// by 2^12 so that lo stays clear of f16's subnormals), because the scalar kernel kept it in f32.  Against
+// 64-bit arithmetic, 2-norm over head_dim 64, f32 out: 1.3e-7 (64 keys causal) to 2.6e-7 (384 keys), the scalar
+// kernel 2.2e-7 to 4.5e-7; the tcgen05 form, whose P is one f16, 1.3e-4 to 2.0e-4 at head_dim 128, here 1.5e-7 to 3.5e-7.
 // Measured: one head of 384 keys, d 128, causal: 12.3 us (tcgen05 form) -> 7.4 us; 1 x 8 heads of 128
 // keys 5.5 us (9.9 us for 300 keys on the tcgen05 form); d 64, 8 x 32 heads of 512 causal: 63 us.
 #include "common.cuh"
@@ -20,7 +22,7 @@
 namespace kaio {
 namespace awarp {
 
-constexpr float P_SHIFT = 12.0f;  // P <= 2^12
+constexpr float P_SCALE = 4096.0f;  // P <= 2^12
 
 __device__ __forceinline__ void cp_async_16_zfill(uint32_t smem, const void* gmem, bool live)
 {
@@ -52,12 +54,34 @@ __device__ __forceinline__ float ex2(float x)
     return y;
 }
 
+// Two f32 operations in one instruction (sm_100).
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
+{
+    float2 d;
+    asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\n"
+        "add.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+
+__device__ __forceinline__ float2 mul2(float2 a, float b)
+{
+    float2 d;
+    asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %4};\n"
+        "mul.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b));
+    return d;
+}
+
 // Two probabilities -> hi and lo f16 pairs.
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo)
 {
     const __half2 h = __floats2half2_rn(a, b);
     const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    const float2 r = add2(make_float2(a, b), make_float2(-f.x, -f.y));
+    const __half2 l = __floats2half2_rn(r.x, r.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
@@ -149,7 +173,8 @@ __global__ void __launch_bounds__(QW* KW * 32) attention_warp_kernel(const AttnP
 #pragma unroll
         for (int j = 0; j < 4; ++j)
             o[i][j] = 0.0f;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
+    float m0 = -INFINITY, m1 = -INFINITY;  // largest raw score q.k of the row
+    float2 l0 = make_float2(0.0f, 0.0f), l1 = l0;
 
     // ldmatrix row addresses of this lane: K: matrices (keys 0-7, d 0-7) (keys 0-7, d 8-15) (keys 8-15,
     // d 0-7) (keys 8-15, d 8-15); V, transposed: (keys 0-7, d 0-7) (keys 8-15, d 0-7) (keys 0-7,
@@ -207,29 +232,37 @@ __global__ void __launch_bounds__(QW* KW * 32) attention_warp_kernel(const AttnP
             x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, d));
             x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, d));
         }
-        const float n0 = fmaxf(m0, x0 * scale_log2), n1 = fmaxf(m1, x1 * scale_log2);
-        const float ref0 = (n0 == -INFINITY ? 0.0f : n0) - P_SHIFT;
-        const float ref1 = (n1 == -INFINITY ? 0.0f : n1) - P_SHIFT;
-        const float al0 = ex2(m0 - P_SHIFT - ref0), al1 = ex2(m1 - P_SHIFT - ref1);
-        m0 = n0;
-        m1 = n1;
-        l0 *= al0;
-        l1 *= al1;
+        // P = 2^((s - m) scale) from the difference of the raw scores: it is exact where P is large, whatever
+        // their size.  With s * scale - n, n the rounded maximum, the exponent was off by the rounding of n:
+        // 2^-21 of P at best, and NaN or nothing from maxima of 2^25 on.
+        x0 = fmaxf(m0, x0);
+        x1 = fmaxf(m1, x1);
+        const float ref0 = x0 == -INFINITY ? 0.0f : x0, ref1 = x1 == -INFINITY ? 0.0f : x1;
+        const float al0 = ex2((m0 - ref0) * scale_log2), al1 = ex2((m1 - ref1) * scale_log2);
+        m0 = x0;
+        m1 = x1;
+        l0 = mul2(l0, al0);
+        l1 = mul2(l1, al1);
 #pragma unroll
         for (int i = 0; i < NO; ++i) {
-            o[i][0] *= al0;
-            o[i][1] *= al0;
-            o[i][2] *= al1;
-            o[i][3] *= al1;
+            const float2 u = mul2(make_float2(o[i][0], o[i][1]), al0);
+            const float2 v = mul2(make_float2(o[i][2], o[i][3]), al1);
+            o[i][0] = u.x;
+            o[i][1] = u.y;
+            o[i][2] = v.x;
+            o[i][3] = v.y;
         }
+        auto prob2 = [&](float& a, float& b, float ref, float2& l) {
+            const float2 e = mul2(add2(make_float2(a, b), make_float2(-ref, -ref)), scale_log2);
+            const float2 pr = mul2(make_float2(ex2(e.x), ex2(e.y)), P_SCALE);
+            l = add2(l, pr);
+            a = pr.x;
+            b = pr.y;
+        };
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
-            s[i][0] = ex2(fmaf(s[i][0], scale_log2, -ref0));
-            s[i][1] = ex2(fmaf(s[i][1], scale_log2, -ref0));
-            s[i][2] = ex2(fmaf(s[i][2], scale_log2, -ref1));
-            s[i][3] = ex2(fmaf(s[i][3], scale_log2, -ref1));
-            l0 += s[i][0] + s[i][1];
-            l1 += s[i][2] + s[i][3];
+            prob2(s[i][0], s[i][1], ref0, l0);
+            prob2(s[i][2], s[i][3], ref1, l1);
         }
 #pragma unroll
         for (int i = 0; i < NS / 2; ++i) {
@@ -254,10 +287,11 @@ __global__ void __launch_bounds__(QW* KW * 32) attention_warp_kernel(const AttnP
         slot = slot + 1 == ST ? 0 : slot + 1;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    float sum0 = l0.x + l0.y, sum1 = l1.x + l1.y;
 #pragma unroll
     for (int d = 1; d < 4; d <<= 1) {
-        l0 += __shfl_xor_sync(0xffffffffu, l0, d);
-        l1 += __shfl_xor_sync(0xffffffffu, l1, d);
+        sum0 += __shfl_xor_sync(0xffffffffu, sum0, d);
+        sum1 += __shfl_xor_sync(0xffffffffu, sum1, d);
     }
     auto inverse = [](float l) { return l > 0.0f ? 1.0f / l : 0.0f; };
     auto store2 = [&](uint32_t row, uint32_t col, float x, float y) {
@@ -268,7 +302,7 @@ __global__ void __launch_bounds__(QW* KW * 32) attention_warp_kernel(const AttnP
             *reinterpret_cast<float2*>(reinterpret_cast<float*>(p.out) + idx) = make_float2(x, y);
     };
     if (KW == 1) {
-        const float i0 = inverse(l0), i1 = inverse(l1);
+        const float i0 = inverse(sum0), i1 = inverse(sum1);
 #pragma unroll
         for (int i = 0; i < NO; ++i) {
             if (row0 < p.seq_q)
@@ -291,9 +325,9 @@ __global__ void __launch_bounds__(QW* KW * 32) attention_warp_kernel(const AttnP
         }
         if (t == 0) {
             ml[(kw * 16 + g) * 2] = m0;
-            ml[(kw * 16 + g) * 2 + 1] = l0;
+            ml[(kw * 16 + g) * 2 + 1] = sum0;
             ml[(kw * 16 + g + 8) * 2] = m1;
-            ml[(kw * 16 + g + 8) * 2 + 1] = l1;
+            ml[(kw * 16 + g + 8) * 2 + 1] = sum1;
         }
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < 16 * D / 2; i += C::THREADS) {
@@ -306,7 +340,7 @@ __global__ void __launch_bounds__(QW* KW * 32) attention_warp_kernel(const AttnP
             float l = 0.0f, x = 0.0f, y = 0.0f;
 #pragma unroll
             for (int w = 0; w < KW; ++w) {
-                const float f = ex2(ml[(w * 16 + r) * 2] - ref);
+                const float f = ex2((ml[(w * 16 + r) * 2] - ref) * scale_log2);
                 const float2 v = *reinterpret_cast<const float2*>(part + (w * 16 + r) * PITCH + c);
                 l += f * ml[(w * 16 + r) * 2 + 1];
                 x += f * v.x;
