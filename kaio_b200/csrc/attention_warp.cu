@@ -15,6 +15,8 @@
 // kernel 2.2e-7 to 4.5e-7; the tcgen05 form, whose P is one f16, 1.3e-4 to 2.0e-4 at head_dim 128, here 1.5e-7 to 3.5e-7.
 // Measured: one head of 384 keys, d 128, causal: 12.3 us (tcgen05 form) -> 7.4 us; 1 x 8 heads of 128
 // keys 5.5 us (9.9 us for 300 keys on the tcgen05 form); d 64, 8 x 32 heads of 512 causal: 63 us.
+#include <cfloat>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "mma_sync.cuh"
@@ -75,6 +77,16 @@ __device__ __forceinline__ float2 mul2(float2 a, float b)
     return d;
 }
 
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\n"
+        "fma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
 // Two probabilities -> hi and lo f16 pairs.
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo)
 {
@@ -84,6 +96,30 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
     const __half2 l = __floats2half2_rn(r.x, r.y);
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// One row of the output by the plain sums, two columns: what the product of P's halves cannot give.  An
+// infinite value meets lo halves that are negative or zero, and, in its stage, masked keys of weight zero.
+template <int D>
+__device__ __forceinline__ float2 plain_output(const __half* q, const __half* k, uint64_t k_row, const __half* v,
+                                               uint64_t v_row, uint32_t keys, float scale_log2, float m, float l)
+{
+    float2 sum = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+    for (uint32_t j = 0; j < keys; ++j, k += k_row, v += v_row) {
+        float dot = 0.0f;
+#pragma unroll 1
+        for (int d = 0; d < D; d += 2) {
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(q + d));
+            const float2 b = __half22float2(*reinterpret_cast<const __half2*>(k + d));
+            dot = fmaf(a.x, b.x, fmaf(a.y, b.y, dot));
+        }
+        const float w = P_SCALE * ex2((dot - m) * scale_log2);
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(v));
+        sum.x = fmaf(w, f.x, sum.x);
+        sum.y = fmaf(w, f.y, sum.y);
+    }
+    return make_float2(sum.x / l, sum.y / l);
 }
 
 // QW warps along the query rows (16 each), KW groups of them along the keys, BKV keys per stage, ST
@@ -294,6 +330,12 @@ __global__ void __launch_bounds__(QW* KW * 32) attention_warp_kernel(const AttnP
         sum1 += __shfl_xor_sync(0xffffffffu, sum1, d);
     }
     auto inverse = [](float l) { return l > 0.0f ? 1.0f / l : 0.0f; };
+    // not finite although the row's scores were (l is)
+    auto lost = [](float x, float l) { return !(fabsf(x) <= FLT_MAX) && l > 0.0f && l <= FLT_MAX; };
+    auto plain2 = [&](uint32_t row, uint32_t col, float m, float l) {
+        return plain_output<D>(p.q + b * p.q_batch + h * p.q_head + row * p.q_row, kbase, p.k_row, vbase + col,
+                               p.v_row, p.causal && row + 1 < p.seq_k ? row + 1 : p.seq_k, scale_log2, m, l);
+    };
     auto store2 = [&](uint32_t row, uint32_t col, float x, float y) {
         const size_t idx = b * p.o_batch + h * p.o_head + (size_t)row * p.o_row + col;
         if (p.out_f16)
@@ -309,6 +351,24 @@ __global__ void __launch_bounds__(QW* KW * 32) attention_warp_kernel(const AttnP
                 store2(row0, i * 8 + 2 * t, o[i][0] * i0, o[i][1] * i0);
             if (row1 < p.seq_q)
                 store2(row1, i * 8 + 2 * t, o[i][2] * i1, o[i][3] * i1);
+        }
+        float2 za = make_float2(0.0f, 0.0f), zb = za;  // NaN if an output of the row is not finite
+#pragma unroll
+        for (int i = 0; i < NO; ++i) {
+            za = fma2(make_float2(o[i][0], o[i][1]), make_float2(0.0f, 0.0f), za);
+            zb = fma2(make_float2(o[i][2], o[i][3]), make_float2(0.0f, 0.0f), zb);
+        }
+        const float z0 = za.x + za.y, z1 = zb.x + zb.y;
+        if (lost(z0, sum0) || lost(z1, sum1)) {
+#pragma unroll 1
+            for (uint32_t i = 0; i < 2 * NO; ++i) {
+                const bool upper = i >= NO;
+                const uint32_t row = upper ? row1 : row0, col = (upper ? i - NO : i) * 8 + 2 * t;
+                if (row < p.seq_q && lost(upper ? z1 : z0, upper ? sum1 : sum0)) {
+                    const float2 v = plain2(row, col, upper ? m1 : m0, upper ? sum1 : sum0);
+                    store2(row, col, v.x, v.y);
+                }
+            }
         }
     } else {
         // ---- the groups' partial results, in ascending group order
@@ -330,25 +390,47 @@ __global__ void __launch_bounds__(QW* KW * 32) attention_warp_kernel(const AttnP
             ml[(kw * 16 + g + 8) * 2 + 1] = sum1;
         }
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < 16 * D / 2; i += C::THREADS) {
-            const uint32_t r = i / (D / 2), c = (i % (D / 2)) * 2;
-            float m = -INFINITY;
+        // outputs (row, col) and (row, col + 1) of the CTA's 16 rows
+        auto merged = [&](uint32_t row, uint32_t col, float& m, float& l) {
+            m = -INFINITY;
 #pragma unroll
             for (int w = 0; w < KW; ++w)
-                m = fmaxf(m, ml[(w * 16 + r) * 2]);
+                m = fmaxf(m, ml[(w * 16 + row) * 2]);
             const float ref = m == -INFINITY ? 0.0f : m;
-            float l = 0.0f, x = 0.0f, y = 0.0f;
+            float x = 0.0f, y = 0.0f;
+            l = 0.0f;
 #pragma unroll
             for (int w = 0; w < KW; ++w) {
-                const float f = ex2((ml[(w * 16 + r) * 2] - ref) * scale_log2);
-                const float2 v = *reinterpret_cast<const float2*>(part + (w * 16 + r) * PITCH + c);
-                l += f * ml[(w * 16 + r) * 2 + 1];
+                const float f = ex2((ml[(w * 16 + row) * 2] - ref) * scale_log2);
+                const float2 v = *reinterpret_cast<const float2*>(part + (w * 16 + row) * PITCH + col);
+                l += f * ml[(w * 16 + row) * 2 + 1];
                 x += f * v.x;
                 y += f * v.y;
             }
             const float inv = inverse(l);
+            return make_float2(x * inv, y * inv);
+        };
+        constexpr uint32_t PAIRS = 16 * D / 2;
+        bool any_lost = false;
+        float m, l;
+#pragma unroll
+        for (uint32_t i = threadIdx.x; i < PAIRS; i += C::THREADS) {
+            const uint32_t r = i / (D / 2), c = (i % (D / 2)) * 2;
+            const float2 v = merged(r, c, m, l);
+            any_lost |= lost(v.x + v.y, l);
             if (q0 + r < p.seq_q)
-                store2(q0 + r, c, x * inv, y * inv);
+                store2(q0 + r, c, v.x, v.y);
+        }
+        if (any_lost) {
+#pragma unroll 1
+            for (uint32_t i = threadIdx.x; i < PAIRS; i += C::THREADS) {
+                const uint32_t r = i / (D / 2), c = (i % (D / 2)) * 2;
+                const float2 v = merged(r, c, m, l);
+                if (q0 + r < p.seq_q && lost(v.x + v.y, l)) {
+                    const float2 w = plain2(q0 + r, c, m, l);
+                    store2(q0 + r, c, w.x, w.y);
+                }
+            }
         }
     }
 }

@@ -1,5 +1,5 @@
 """Attention with values at the ends of the f16 range, on the warp-MMA and the one-row kernels: scores far
-beyond what an exponent holds, and rows whose result is known to the last bit."""
+beyond what an exponent holds, rows whose result is known to the last bit, infinities and NaN."""
 import numpy as np
 import pytest
 import torch
@@ -52,3 +52,49 @@ def test_a_row_that_sees_one_key_is_its_value(seq, d):
     ops.attention_tc_causal(device(), q, k, v, out, seq, seq, d, d)
     assert ops.last_variant() == "attention_warp_mma"
     assert torch.equal(out[:d], v[:d].float())
+
+
+@pytest.mark.parametrize("special", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("b,h,sq,sk,d", SHAPES)
+def test_special_values(oracle, b, h, sq, sk, d, special):
+    """One element of one key, and of one value, of head 0 of batch 0.  What the oracle makes non-finite is
+    non-finite of the same kind, what has weight zero or belongs to another head stays finite and right."""
+    rng = np.random.default_rng(sk)
+    q, k, v = [rng.standard_normal((b, n, h, d)).astype(np.float16) for n in (sq, sk, sk)]
+    q[:, :, 0, 5] = np.abs(q[:, :, 0, 5]) + np.float16(0.1)
+    for t, name in ((k, "k"), (v, "v")):
+        clean = t[0, sk // 2, 0, 5]
+        t[0, sk // 2, 0, 5] = special
+        got = attend(q, k, v, b, h, sq, sk, d, False)
+        t_q, t_k, t_v = [np.ascontiguousarray(x.transpose(0, 2, 1, 3)) for x in (q, k, v)]
+        for bi in range(b):
+            for hi in range(h):
+                with np.errstate(all="ignore"):
+                    want = oracle.attention(t_q[bi, hi], t_k[bi, hi], t_v[bi, hi], sq, sk, d, d)
+                want = np.asarray(want, dtype=np.float64).reshape(sq, d)
+                if name == "k" and bi == 0 and hi == 0 and special != float("-inf"):
+                    assert np.isnan(got[bi, :, hi]).all()  # inf - inf or NaN in every row
+                    continue
+                same = np.isfinite(want)
+                assert np.array_equal(np.isnan(got[bi, :, hi]), np.isnan(want))
+                assert np.array_equal(got[bi, :, hi][~same], want[~same], equal_nan=True)
+                # one f16 rounding beside the f32 sums
+                assert np.all(np.abs(got[bi, :, hi][same] - want[same]) <= 2.0 ** -10 * np.abs(want[same]) + 2e-5)
+        t[0, sk // 2, 0, 5] = clean
+
+
+@pytest.mark.parametrize("special", [float("nan"), float("inf")])
+@pytest.mark.parametrize("b,h,sq,sk,d", [s for s in SHAPES if s[2] > 1])
+def test_rows_that_do_not_see_a_value_are_not_touched_by_it(b, h, sq, sk, d, special):
+    """Causal: the key sits in the middle of a 16- and of a 64-key stage, so earlier rows meet it masked."""
+    rng = np.random.default_rng(sk + d)
+    q, k, v = [rng.standard_normal((b, n, h, d)).astype(np.float16) for n in (sq, sk, sk)]
+    clean = attend(q, k, v, b, h, sq, sk, d, True)
+    key = 21
+    v[0, key, 0, 5] = special
+    got = attend(q, k, v, b, h, sq, sk, d, True)
+    seen = np.zeros(got.shape, bool)
+    seen[0, key:, 0, 5] = True
+    assert np.array_equal(got[seen], np.full(seen.sum(), special), equal_nan=True)
+    # the masked meeting is summed once more in another order: one f16 rounding and f32 sums apart
+    assert np.all(np.abs(got - clean)[~seen] <= 2.0 ** -10 * np.abs(clean[~seen]) + 2e-5)
