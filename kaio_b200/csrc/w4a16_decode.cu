@@ -55,6 +55,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "unit_ranges.cuh"
 
 namespace kaio {
 namespace w4dec {
@@ -106,6 +107,7 @@ struct Params {
     uint32_t m, n, k;
     uint32_t num_kb;       // ceil(K / 256)
     uint32_t num_tiles;    // ceil(N / 128)
+    UnitRanges ranges;     // of the num_tiles * num_kb units
     uint32_t* status;
 };
 
@@ -223,23 +225,6 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
         : "memory");
 }
 
-// First unit of CTA c when `units` units are cut into `grid` contiguous ranges: c * units / grid in
-// 32-bit steps (grid^2 is below 2^32).  As 64-bit quotients the ranges cost 1 us of the 128 of the 70B FFN at M = 16: they stand
-// in front of the first load and in the chain behind the last product.
-__device__ __forceinline__ uint32_t range_begin(uint32_t c, uint32_t units, uint32_t grid)
-{
-    const uint32_t len = units / grid, rem = units - len * grid;
-    return c * len + c * rem / grid;
-}
-
-// The CTA whose range holds unit u.
-__device__ __forceinline__ uint32_t owner_of(uint32_t u, uint32_t units, uint32_t grid)
-{
-    if (__umulhi(units, grid) == 0)  // (u + 1) * grid fits 32 bits
-        return ((u + 1) * grid - 1) / units;
-    return (uint32_t)((((uint64_t)u + 1) * grid - 1) / units);
-}
-
 // The producer and the MMA issuer poll (their reaction time is on the critical path of every
 // stage); the many dequantising and epilogue warps park in try_wait and leave the issue slots
 // to the arithmetic.
@@ -318,9 +303,8 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmap_w,
         trace_ptr[47 * 8 + 4] = clock64();
     }
 #endif
-    const uint32_t units = p.num_tiles * p.num_kb;
-    const uint32_t u_begin = range_begin(blockIdx.x, units, gridDim.x);
-    uint32_t u_end = range_begin(blockIdx.x + 1, units, gridDim.x);
+    const uint32_t u_begin = p.ranges.begin(blockIdx.x);
+    uint32_t u_end = p.ranges.begin(blockIdx.x + 1);
     if (!layout_ok) {
         // never seen (the dynamic window starts 1024-aligned when a kernel has no static shared
         // memory); reported instead of assumed
@@ -696,8 +680,8 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmap_w,
                 // cumulative).  Separate fences around a relaxed atomic are three dependent
                 // round trips to L2 instead of one, in the tail of every CTA.
                 named_barrier(2, 128);
-                const uint32_t c_first = owner_of(tile * p.num_kb, units, gridDim.x);
-                const uint32_t c_last = owner_of(tile * p.num_kb + p.num_kb - 1, units, gridDim.x);
+                const uint32_t c_first = p.ranges.owner(tile * p.num_kb);
+                const uint32_t c_last = p.ranges.owner(tile * p.num_kb + p.num_kb - 1);
                 if (tid == 0) {
                     uint32_t prev;
                     asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
@@ -718,8 +702,7 @@ w4a16_decode_kernel(const __grid_constant__ CUtensorMap tmap_w,
 #pragma unroll 2  // two contributors' loads in flight
                     for (uint32_t c = c_first; c <= c_last; ++c) {
                         // the tile opens c's range unless an earlier one does
-                        const uint32_t cslot =
-                            range_begin(c, units, gridDim.x) >= tile * p.num_kb ? 0u : 1u;
+                        const uint32_t cslot = p.ranges.begin(c) >= tile * p.num_kb ? 0u : 1u;
                         const float* src =
                             p.partials + ((size_t)(c * 2 + cslot) * PARTIAL_FLOATS) + tid * 16;
 #pragma unroll
@@ -832,6 +815,7 @@ cudaError_t launch_w4a16_decode_tc(const DeviceCtx& ctx, const __half* x, const 
     p.num_tiles = (n + BN - 1) / BN;
     p.status = ctx.status;
     const uint32_t grid = decode_grid(ctx, n, k);
+    p.ranges = unit_ranges(p.num_tiles * p.num_kb, grid);
 
     // Programmatic dependent launch: this launch may begin (weight prefetch, first
     // dequantisation) while the kernel in front of it in the stream drains; it reads the

@@ -33,6 +33,7 @@
 // on timing.
 #include "common.cuh"
 #include "kernels.h"
+#include "unit_ranges.cuh"
 
 namespace kaio {
 namespace w4f {
@@ -97,6 +98,7 @@ struct Params {
     // into gridDim contiguous ranges; a tile that a cut splits is summed from f32 partial
     // tiles in a workspace by the last CTA to arrive, in ascending CTA order (deterministic).
     int streamk;
+    UnitRanges ranges;
     float4* partials;    // [grid][2][NROWS / 4][128 columns] float4 (4 rows of one column)
     uint32_t* counters;  // [tiles], zero between launches
     uint32_t* status;
@@ -120,23 +122,6 @@ __device__ __forceinline__ void named_barrier(uint32_t id, uint32_t count)
 __device__ __forceinline__ void fence_acq_rel_gpu()
 {
     asm volatile("fence.acq_rel.gpu;" ::: "memory");
-}
-
-// First unit of CTA c when `units` units are cut into `grid` contiguous ranges: c * units / grid in
-// 32-bit steps (grid^2 is below 2^32).  As 64-bit quotients the ranges cost 2 us of the 154 of 28672 x 8192 at M = 250: they stand
-// in front of the first load and in the chain behind the last product.
-__device__ __forceinline__ uint32_t range_begin(uint32_t c, uint32_t units, uint32_t grid)
-{
-    const uint32_t len = units / grid, rem = units - len * grid;
-    return c * len + c * rem / grid;
-}
-
-// The CTA whose range holds unit u.
-__device__ __forceinline__ uint32_t owner_of(uint32_t u, uint32_t units, uint32_t grid)
-{
-    if (__umulhi(units, grid) == 0)  // (u + 1) * grid fits 32 bits
-        return ((u + 1) * grid - 1) / units;
-    return (uint32_t)((((uint64_t)u + 1) * grid - 1) / units);
 }
 
 struct TensorMaps {
@@ -247,12 +232,11 @@ w4a16_fused_kernel(const __grid_constant__ TensorMaps maps, const Params p)
         n0 = (r / tiles_m) * BN;
     };
 
-    const uint32_t units = num_tiles * num_kb;
     auto seg_begin = [&]() {
         SegIter it;
         it.tile = blockIdx.x;
-        it.u = range_begin(blockIdx.x, units, gridDim.x);
-        it.u1 = range_begin(blockIdx.x + 1, units, gridDim.x);
+        it.u = p.ranges.begin(blockIdx.x);
+        it.u1 = p.ranges.begin(blockIdx.x + 1);
         return it;
     };
     auto seg_next = [&](SegIter& it, Seg& g) {
@@ -471,7 +455,7 @@ w4a16_fused_kernel(const __grid_constant__ TensorMaps maps, const Params p)
         const uint32_t q = warp & 3u;
         const uint32_t tid = q * 32 + lane;  // weight column inside the tile = TMEM lane
         constexpr uint32_t PART_F4 = (NROWS / 4) * BN;  // float4 per parked partial tile
-        const uint32_t first_tile = range_begin(blockIdx.x, units, gridDim.x) / num_kb;
+        const uint32_t first_tile = p.ranges.begin(blockIdx.x) / num_kb;
         uint32_t local_tile = 0;
         SegIter it = seg_begin();
         Seg g;
@@ -494,20 +478,28 @@ w4a16_fused_kernel(const __grid_constant__ TensorMaps maps, const Params p)
                 const uint32_t d_lo = p.scatter_cols ? col / p.scatter_cols : 0u;
                 const uint32_t d_hi = p.scatter_cols ? d_lo + 1u : (p.num_copies ? p.num_copies : 1u);
                 const uint32_t dcol = p.scatter_cols ? col - d_lo * p.scatter_cols : col;
+                // The rows walk by additions.  As 32 products with the row stride the addresses were kept
+                // over the loop of destinations, on the stack: 900 to 1100 bytes of spills (us with them /
+                // without, M x K x N: 64 x 4096 x 4096 20.6 / 16.1, 200 x 4096 x 11008 41.4 / 31.9, 512 x 4096 x
+                // 4096 30.1 / 24.3, 250 x 28672 x 8192 134 / 121; three 8192 -> 1024 ones at 500 rows 69 / 34).
+                const uint32_t row0 = m0 + c * 32;
+                const uint32_t rows = p.m - row0 < 32u ? p.m - row0 : 32u;
+                const size_t ld = p.num_copies ? (size_t)p.ld : (size_t)p.n;
+#pragma unroll 1
                 for (uint32_t d = d_lo; d < d_hi; ++d) {
                     void* const dst = p.num_copies ? p.copies[d] : p.probs[prob].out;
-                    const size_t ld = p.num_copies ? (size_t)p.ld : (size_t)p.n;
+                    if (p.out_f16) {
+                        __half* o = reinterpret_cast<__half*>(dst) + (size_t)row0 * ld + dcol;
 #pragma unroll
-                    for (uint32_t i = 0; i < 32; ++i) {
-                        const uint32_t rr = m0 + c * 32 + i;
-                        if (rr < p.m) {
-                            const size_t idx = (size_t)rr * ld + dcol;
-                            if (p.out_f16)
-                                reinterpret_cast<__half*>(dst)[idx] =
-                                    __float2half_rn(__uint_as_float(r[i]));
-                            else
-                                reinterpret_cast<float*>(dst)[idx] = __uint_as_float(r[i]);
-                        }
+                        for (uint32_t i = 0; i < 32; ++i, o += ld)
+                            if (i < rows)
+                                *o = __float2half_rn(__uint_as_float(r[i]));
+                    } else {
+                        float* o = reinterpret_cast<float*>(dst) + (size_t)row0 * ld + dcol;
+#pragma unroll
+                        for (uint32_t i = 0; i < 32; ++i, o += ld)
+                            if (i < rows)
+                                *o = __uint_as_float(r[i]);
                     }
                 }
             };
@@ -552,8 +544,8 @@ w4a16_fused_kernel(const __grid_constant__ TensorMaps maps, const Params p)
                                        __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
             }
             release_d();
-            const uint32_t c_first = owner_of(g.tile * num_kb, units, gridDim.x);
-            const uint32_t c_last = owner_of(g.tile * num_kb + num_kb - 1, units, gridDim.x);
+            const uint32_t c_first = p.ranges.owner(g.tile * num_kb);
+            const uint32_t c_last = p.ranges.owner(g.tile * num_kb + num_kb - 1);
             // one thread fences for the four warps: the barrier in front orders their parked
             // stores before its release fence, the barrier behind orders its acquire fence before
             // their loads
@@ -583,8 +575,7 @@ w4a16_fused_kernel(const __grid_constant__ TensorMaps maps, const Params p)
 #pragma unroll 2  // two contributors' loads in flight
                 for (uint32_t cc = c_first; cc <= c_last; ++cc) {  // ascending: a fixed order
                     // the tile opens cc's range unless an earlier one does
-                    const uint32_t cslot =
-                        range_begin(cc, units, gridDim.x) >= g.tile * num_kb ? 0u : 1u;
+                    const uint32_t cslot = p.ranges.begin(cc) >= g.tile * num_kb ? 0u : 1u;
                     const float4* src = p.partials + (size_t)(cc * 2 + cslot) * PART_F4 + tid;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
@@ -739,14 +730,15 @@ static cudaError_t launch_fused_n(const DeviceCtx& ctx, const __half* x, const D
     p.status = ctx.status;
     const uint32_t tiles = ((m + NROWS - 1) / NROWS) * ((n + BN - 1) / BN) * (uint32_t)num_probs;
     uint32_t grid = tiles < (uint32_t)ctx.num_sms ? tiles : (uint32_t)ctx.num_sms;
+    const uint32_t units = tiles * ((k + BKS - 1) / BKS);
     p.streamk = 0;
     p.partials = reinterpret_cast<float4*>(workspace);
     p.counters = counters;
     if (workspace != nullptr && counters != nullptr && fused_plan(ctx, num_probs, m, n, k).streamk) {
         p.streamk = 1;
-        const uint32_t units = tiles * ((k + BKS - 1) / BKS);
         grid = units < (uint32_t)ctx.num_sms ? units : (uint32_t)ctx.num_sms;
     }
+    p.ranges = unit_ranges(units, grid);
     static bool attr_set[64] = {};
     if (!attr_set[ctx.device]) {
         err = cudaFuncSetAttribute(w4a16_fused_kernel<NROWS, BKS>,
