@@ -114,13 +114,17 @@ struct AnyBuf {  // f16 or f32, as void*
     }
 };
 
+// An int or whatever stands for one (a numpy integer, an integer tensor of one element), modulo 2^64.
 unsigned long long unpack_int(PyObject* o, const char* what)
 {
-    const unsigned long long v = PyLong_Check(o) ? PyLong_AsUnsignedLongLongMask(o) : 0;
-    if (!PyLong_Check(o)) {
-        PyErr_Format(PyExc_TypeError, "%s: expected an int, got %s", what, Py_TYPE(o)->tp_name);
+    PyObject* i = PyNumber_Index(o);
+    if (!i) {
+        if (PyErr_ExceptionMatches(PyExc_TypeError))
+            PyErr_Format(PyExc_TypeError, "%s: expected an int, got %s", what, Py_TYPE(o)->tp_name);
         throw ArgError();
     }
+    const unsigned long long v = PyLong_AsUnsignedLongLongMask(i);
+    Py_DECREF(i);
     return v;
 }
 
