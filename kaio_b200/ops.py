@@ -79,6 +79,14 @@ def probe_int8_mma_rate(device: KaioDevice, iters: int) -> int:
     return int(ops_count.value)
 
 
+def _addresses(ptrs, world):
+    """The addresses as ints; a list longer than the ranks it is for is a mistake of the caller."""
+    addresses = [int(p) for p in ptrs]
+    if len(addresses) > world:
+        raise IndexError(f"{len(addresses)} device addresses for {world} ranks")
+    return addresses
+
+
 # ------------------------------------------------------------------ W8A8
 
 def matmul_int8(device, a, b, c, scale, m, n, k):
@@ -135,7 +143,7 @@ def matmul_int4_allgather(device, a, b_packed_shard, scales_shard, out_ptrs, out
     """Extension: this rank's column shard of a W4A16 GEMM, stored by the kernel into every rank's
     f16 ``[m, n_total]`` buffer.  ``out_ptrs`` are ``world`` device addresses as mapped in this
     process (e.g. ``torch.distributed._symmetric_memory`` ``buffer_ptrs``)."""
-    _native.matmul_int4_allgather(device, a, b_packed_shard, scales_shard, [int(p) for p in out_ptrs],
+    _native.matmul_int4_allgather(device, a, b_packed_shard, scales_shard, _addresses(out_ptrs, world),
                                   out_numel, world, rank, m, n_total, k, group_size)
 
 
@@ -144,7 +152,7 @@ def matmul_int4_allgather_multicast(device, a, b_packed_shard, scales_shard, out
     """Extension: :func:`matmul_int4_allgather` whose large-``m`` kernel writes each output block once
     through ``multicast_out``, the NVLink multicast address of the ``[m, n_total]`` output
     (``multimem.st``; the switch delivers it to every rank)."""
-    _native.matmul_int4_allgather_multicast(device, a, b_packed_shard, scales_shard, [int(p) for p in out_ptrs],
+    _native.matmul_int4_allgather_multicast(device, a, b_packed_shard, scales_shard, _addresses(out_ptrs, world),
                                             out_numel, int(multicast_out), world, rank, m, n_total, k,
                                             group_size)
 
@@ -165,7 +173,7 @@ def matmul_int4_peer_partials(device, a, b_packed, scales, slot_ptrs, slot_numel
     addresses as mapped in this process, each f32 ``[world][m][cols]``).  ``scatter=False``: the
     whole partial to every rank (``cols = n``); ``scatter=True``: column block ``d`` to rank ``d``
     only (``cols = n / world``)."""
-    _native.matmul_int4_peer_partials(device, a, b_packed, scales, [int(p) for p in slot_ptrs], slot_numel,
+    _native.matmul_int4_peer_partials(device, a, b_packed, scales, _addresses(slot_ptrs, world), slot_numel,
                                       world, rank, 1 if scatter else 0, m, n, k, group_size)
 
 

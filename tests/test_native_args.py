@@ -21,3 +21,12 @@ def test_integers_of_other_types_are_integers():
         assert not isinstance(e.value, TypeError), e.value
     for bad in (0.0, "0", None):
         refused(TypeError, ops.selftest_bounded_wait, bad, match="budget_us: expected an int")
+
+
+def test_more_addresses_than_ranks_are_refused():
+    t = torch.zeros(1)
+    for fn, args in [
+            (ops.matmul_int4_allgather, (t, t, t, [1, 2, 3], 8, 2, 0, 1, 16, 128, 128)),
+            (ops.matmul_int4_allgather_multicast, (t, t, t, range(1, 11), 8, 4096, 8, 0, 1, 64, 128, 128)),
+            (ops.matmul_int4_peer_partials, (t, t, t, [1, 2], 8, 1, 0, False, 1, 16, 128, 128))]:
+        refused(IndexError, fn, *args, match="device addresses for")
