@@ -208,6 +208,14 @@ def allreduce_multimem_f32(device, multicast_in, multicast_out, numel, rows, col
 
 # ------------------------------------------------------------------ fused QKV
 
+def _scale_len(*scales):
+    """Length that the three column-scale tensors have in common."""
+    for name, t in zip(("scale_q", "scale_k", "scale_v"), scales):
+        if not isinstance(t, torch.Tensor):
+            raise TypeError(f"{name}: expected a torch.Tensor, got {type(t).__name__}")
+    return min(t.numel() for t in scales)
+
+
 def qkv_project_int8(device, x, w_q, w_k, w_v, scale_q, scale_k, scale_v, q_out, k_out, v_out, m, n, k):
     """``kaio_ops::qkv_project_int8`` (kaio-ops/src/qkv_project_int8_kernel.rs:2008-2064).
 
@@ -215,7 +223,7 @@ def qkv_project_int8(device, x, w_q, w_k, w_v, scale_q, scale_k, scale_v, q_out,
     extension.
     """
     if isinstance(scale_q, torch.Tensor):
-        scale_len = min(scale_q.numel(), scale_k.numel(), scale_v.numel())
+        scale_len = _scale_len(scale_q, scale_k, scale_v)
         _native.qkv_project_int8_colscale(device, x, w_q, w_k, w_v, scale_q, scale_k, scale_v, scale_len, q_out,
                                           k_out, v_out, m, n, k)
         return
@@ -226,7 +234,7 @@ def qkv_project_w8a8(device, x, w_q, w_k, w_v, scale_q, scale_k, scale_v, q_out,
     """Extension: the W8A8 fused QKV projection -- ``x`` (f16) quantised per row to s8 on the fly,
     s32 accumulation on the INT8 tensor pipe, per-row x per-column scales, f16 outputs.
     ``scale_*`` are float32 tensors of length ``n``."""
-    scale_len = min(scale_q.numel(), scale_k.numel(), scale_v.numel())
+    scale_len = _scale_len(scale_q, scale_k, scale_v)
     _native.qkv_project_w8a8(device, x, w_q, w_k, w_v, scale_q, scale_k, scale_v, scale_len, q_out, k_out,
                              v_out, m, n, k)
 

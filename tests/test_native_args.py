@@ -30,3 +30,10 @@ def test_more_addresses_than_ranks_are_refused():
             (ops.matmul_int4_allgather_multicast, (t, t, t, range(1, 11), 8, 4096, 8, 0, 1, 64, 128, 128)),
             (ops.matmul_int4_peer_partials, (t, t, t, [1, 2], 8, 1, 0, False, 1, 16, 128, 128))]:
         refused(IndexError, fn, *args, match="device addresses for")
+
+
+def test_a_scale_that_is_no_tensor_is_named():
+    t, s = torch.zeros(1), torch.ones(1)
+    refused(TypeError, ops.qkv_project_w8a8, t, t, t, t, 0.5, s, s, t, t, t, 1, 16, 32, match="scale_q: expected a torch.Tensor")
+    refused(TypeError, ops.qkv_project_w8a8, t, t, t, t, s, s, None, t, t, t, 1, 16, 32, match="scale_v: expected a torch.Tensor")
+    refused(TypeError, ops.qkv_project_int8, t, t, t, t, s, 0.5, s, t, t, t, 1, 16, 32, match="scale_k: expected a torch.Tensor")
