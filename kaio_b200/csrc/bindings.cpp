@@ -26,7 +26,8 @@
 namespace {
 
 PyObject* g_from_code = nullptr;  // kaio_b200.errors.from_code
-PyObject *g_ordinal = nullptr, *g_stream = nullptr, *g_cuda_stream = nullptr;  // interned names
+PyObject* g_device_type = nullptr;  // kaio_b200.ops.KaioDevice
+PyObject *g_ordinal = nullptr, *g_stream = nullptr, *g_cuda_stream = nullptr, *g_stream_handle = nullptr;  // names
 
 struct ArgError {};  // a Python exception has been set
 
@@ -171,32 +172,35 @@ struct Ptrs {  // up to eight addresses; the C side rejects a world / num_out ab
 
 // ---------------------------------------------------------------- the call
 // Makes the KaioDevice's device current for the call (restored when it was another one) and finds
-// its stream: the one it was created with, else torch's current stream of that device.
+// its stream: the one it was created with, else torch's current stream of that device.  Another type
+// of device is asked for its stream_handle().
 struct DeviceScope {
     c10::DeviceIndex before, mine;
     void* stream = nullptr;
 
     explicit DeviceScope(PyObject* dev)
     {
-        PyObject* o = PyObject_GetAttr(dev, g_ordinal);
-        if (!o)
-            throw ArgError();
+        PyObject* o = attribute(dev, g_ordinal);
         const long ord = PyLong_AsLong(o);
         Py_DECREF(o);
         if (ord == -1 && PyErr_Occurred())
             throw ArgError();
         mine = (c10::DeviceIndex)ord;
-        PyObject* s = PyObject_GetAttr(dev, g_stream);
-        if (!s)
-            throw ArgError();
-        if (s == Py_None) {
-            stream = c10::cuda::getCurrentCUDAStream(mine).stream();
+        PyObject* handle = nullptr;
+        if (reinterpret_cast<PyObject*>(Py_TYPE(dev)) == g_device_type) {
+            PyObject* s = attribute(dev, g_stream);
+            if (s == Py_None)
+                stream = c10::cuda::getCurrentCUDAStream(mine).stream();
+            else
+                handle = PyObject_GetAttr(s, g_cuda_stream);
+            Py_DECREF(s);
         } else {
-            PyObject* h = PyObject_GetAttr(s, g_cuda_stream);
-            stream = h ? reinterpret_cast<void*>(PyLong_AsUnsignedLongLongMask(h)) : nullptr;
-            Py_XDECREF(h);
+            handle = PyObject_CallMethodNoArgs(dev, g_stream_handle);
         }
-        Py_DECREF(s);
+        if (handle) {
+            stream = reinterpret_cast<void*>(PyLong_AsUnsignedLongLongMask(handle));
+            Py_DECREF(handle);
+        }
         if (PyErr_Occurred())
             throw ArgError();
         before = c10::cuda::current_device();
@@ -207,6 +211,14 @@ struct DeviceScope {
     {
         if (before != mine)
             c10::cuda::set_device(before);
+    }
+
+    static PyObject* attribute(PyObject* o, PyObject* name)
+    {
+        PyObject* v = PyObject_GetAttr(o, name);
+        if (!v)
+            throw ArgError();
+        return v;
     }
 };
 
@@ -373,7 +385,13 @@ PyMODINIT_FUNC PyInit__native()
     g_ordinal = PyUnicode_InternFromString("ordinal");
     g_stream = PyUnicode_InternFromString("_stream");
     g_cuda_stream = PyUnicode_InternFromString("cuda_stream");
-    if (!g_from_code || !g_ordinal || !g_stream || !g_cuda_stream)
+    g_stream_handle = PyUnicode_InternFromString("stream_handle");
+    PyObject* ops = PyImport_ImportModule("kaio_b200.ops");
+    if (!ops)
+        return nullptr;
+    g_device_type = PyObject_GetAttrString(ops, "KaioDevice");
+    Py_DECREF(ops);
+    if (!g_from_code || !g_device_type || !g_ordinal || !g_stream || !g_cuda_stream || !g_stream_handle)
         return nullptr;
     return PyModule_Create(&g_module);
 }

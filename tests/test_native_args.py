@@ -37,3 +37,19 @@ def test_a_scale_that_is_no_tensor_is_named():
     refused(TypeError, ops.qkv_project_w8a8, t, t, t, t, 0.5, s, s, t, t, t, 1, 16, 32, match="scale_q: expected a torch.Tensor")
     refused(TypeError, ops.qkv_project_w8a8, t, t, t, t, s, s, None, t, t, t, 1, 16, 32, match="scale_v: expected a torch.Tensor")
     refused(TypeError, ops.qkv_project_int8, t, t, t, t, s, 0.5, s, t, t, t, 1, 16, 32, match="scale_k: expected a torch.Tensor")
+
+
+def test_a_device_of_another_type_is_asked_for_its_stream():
+    class Pool(ops.KaioDevice):
+        def stream_handle(self):
+            raise KeyError("no stream left")
+
+    class Plain:
+        ordinal = 0
+
+        def stream_handle(self):
+            raise KeyError("no stream left")
+
+    for d in (Pool(0), Plain()):
+        with pytest.raises(KeyError):
+            ops.selftest_bounded_wait(d, 5)
