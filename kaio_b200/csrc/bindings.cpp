@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cstring>
 #include <tuple>
 #include <utility>
 
@@ -38,6 +39,12 @@ const char* dtype_name(c10::ScalarType t)
     case c10::kInt: return "torch.int32";
     case c10::kHalf: return "torch.float16";
     case c10::kFloat: return "torch.float32";
+    case c10::kDouble: return "torch.float64";
+    case c10::kBFloat16: return "torch.bfloat16";
+    case c10::kByte: return "torch.uint8";
+    case c10::kShort: return "torch.int16";
+    case c10::kLong: return "torch.int64";
+    case c10::kBool: return "torch.bool";
     default: return c10::toString(t);
     }
 }
@@ -210,7 +217,7 @@ struct DeviceScope {
     ~DeviceScope()
     {
         if (before != mine)
-            c10::cuda::set_device(before);
+            (void)c10::cuda::MaybeSetDevice(before);  // set_device would throw, out of a destructor
     }
 
     static PyObject* attribute(PyObject* o, PyObject* name)
@@ -222,9 +229,19 @@ struct DeviceScope {
     }
 };
 
+// Held again at the end of the scope, whichever way it is left: what the library throws (memory) is
+// turned into a Python exception further up.
+struct WithoutGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
 PyObject* raise_code(int32_t code)
 {
-    PyObject* e = PyObject_CallFunction(g_from_code, "is", (int)code, kaio_b200_last_error());
+    const char* text = kaio_b200_last_error();
+    PyObject* message = PyUnicode_DecodeUTF8(text, (Py_ssize_t)strlen(text), "replace");  // it may be cut anywhere
+    PyObject* e = message ? PyObject_CallFunction(g_from_code, "iO", (int)code, message) : nullptr;
+    Py_XDECREF(message);
     if (e) {
         PyErr_SetObject(reinterpret_cast<PyObject*>(Py_TYPE(e)), e);
         Py_DECREF(e);
@@ -240,13 +257,14 @@ PyObject* call(Fn fn, const char* const* names, PyObject* const* args, Py_ssize_
         return nullptr;
     }
     try {
-        auto c_args = std::tuple_cat(Kinds::get(args[I + 1], names[I])...);
+        // braces: from left to right, so that the first argument that is wrong is the one reported
+        std::tuple<decltype(Kinds::get(args[I + 1], names[I]))...> each{Kinds::get(args[I + 1], names[I])...};
+        auto c_args = std::apply([](const auto&... a) { return std::tuple_cat(a...); }, each);
         int32_t code;
         {
             DeviceScope scope(args[0]);
-            PyThreadState* ts = PyEval_SaveThread();
+            WithoutGil nogil;
             code = std::apply([&](const auto&... a) { return fn(a..., scope.stream); }, c_args);
-            PyEval_RestoreThread(ts);
         }
         if (code != 0)
             return raise_code(code);

@@ -53,3 +53,9 @@ def test_a_device_of_another_type_is_asked_for_its_stream():
     for d in (Pool(0), Plain()):
         with pytest.raises(KeyError):
             ops.selftest_bounded_wait(d, 5)
+
+
+def test_a_wrong_dtype_is_named_as_torch_names_it():
+    a = torch.zeros(4, dtype=torch.int8)
+    for dtype in (torch.float64, torch.bfloat16, torch.uint8, torch.int16, torch.int64, torch.bool, torch.float32):
+        refused(TypeError, ops.matmul_int8, a.to(dtype), a, a, 1.0, 1, 1, 32, match=f"a: expected dtype torch.int8, got {dtype}")
