@@ -26,6 +26,11 @@
  *     which synchronises the device.  Growth is refused (KAIO_B200_ERR_INVALID_CONFIG) while the
  *     stream is being captured into a CUDA graph, and a graph captured earlier keeps the old
  *     address: run every op once at its largest shape before capturing;
+ *   - kaio_b200_matmul_int4 and its f16, all-gather, peer-partial and no-alloc forms with m <= 16 are
+ *     launched with programmatic stream serialisation and read b_packed and scales (nothing else) without
+ *     waiting for the kernel directly in front on the stream.  A kernel in front that writes these two and
+ *     lets its dependents start early (griddepcontrol.launch_dependents, as these forms themselves do)
+ *     needs another operation or an event between the two;
  *   - return value: KAIO_B200_OK or an error code; kaio_b200_last_error() returns the
  *     calling thread's last message.  For KAIO_B200_ERR_INVALID_CONFIG the message is
  *     the text the reference puts into KaioError::InvalidConfig;

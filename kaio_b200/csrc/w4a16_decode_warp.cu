@@ -25,7 +25,10 @@
 // contiguous range per CTA (two CTAs per SM) and dealt to its eight warps in turn; a tile's partial
 // sums meet in shared memory, and where a range ends inside a tile the CTAs park f32 partials that
 // the last one to arrive adds in ascending CTA order (deterministic; no float atomics).
-// Programmatic dependent launch: what runs before griddepcontrol.wait reads only weights and scales.
+// Programmatic dependent launch: what runs before griddepcontrol.wait reads only weights and scales, and of
+// three matrices not even these.  The early reads save 0.5 to 1 us where calls follow each other (13.6 against
+// 14.4 us for three of 4096 x 4096 at M = 8), but weights or scales that the kernel in front writes would be
+// read too early if it lets its dependents start; a fused QKV call never asked its callers to mind that.
 // Measured (us, tcgen05 form -> this one, weights from HBM), M = 1, K x N: 1024 x 1024 7.1 -> 2.5,
 // 4096 x 4096 13.0 -> 7.8, 28672 x 1024 28.2 -> 10.7, 4096 x 11008 15.1 -> 12.4, 8192 x 28672 41 -> 33.2
 // (3.5 TB/s); three 4096 x 4096 matrices at M = 8 62.7 (f16 copy of the weights, then a GEMM) -> 14.1.
@@ -70,6 +73,7 @@ struct Params {
     uint32_t num_kb;        // units per tile
     uint32_t tiles;         // per weight matrix
     uint32_t per_cta, rem;  // units of all matrices = gridDim.x * per_cta + rem
+    bool weights_wait;      // weights and scales are read only behind the launch in front
 };
 
 // CTA c's range of units: `rem` CTAs of per_cta + 1 units, then CTAs of per_cta.  (With the ranges as
@@ -100,6 +104,14 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait()
 {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Not a read-only (nc) load: the compiler may move such a one over the wait for the launch in front.
+__device__ __forceinline__ uint32_t load_scale(const unsigned short* p)
+{
+    unsigned short v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return v;
 }
 
 // (w & mask) ^ flip in one instruction
@@ -224,7 +236,7 @@ __global__ void __launch_bounds__(NUM_THREADS, CTAS_PER_SM) w4a16_decode_warp_ke
     auto fetch_scales = [&]() {
 #pragma unroll
         for (int j = 0; j < 2 * TC; ++j)
-            sc[j] = (n_mask >> j & 1u) ? (uint32_t)__ldg(n_scale + j * 8) : 0u;
+            sc[j] = (n_mask >> j & 1u) ? load_scale(n_scale + j * 8) : 0u;
     };
     uint4 xr[NB][4];  // row g (and g + 8): the 32 k of this lane
     auto fetch_x = [&]() {
@@ -241,6 +253,8 @@ __global__ void __launch_bounds__(NUM_THREADS, CTAS_PER_SM) w4a16_decode_warp_ke
         a_setup();
         n_setup();
     }
+    if (p.weights_wait)
+        asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
     for (uint32_t i = 0; i < AHEAD; ++i) {
 #pragma unroll
@@ -500,6 +514,7 @@ cudaError_t launch_w4a16_decode(const DeviceCtx& ctx, const __half* x, const DqP
         grid = (uint32_t)ctx.num_sms * CTAS_PER_SM;
     p.per_cta = units / grid;
     p.rem = units % grid;
+    p.weights_wait = num_probs == 3;
 
     // Programmatic dependent launch: this launch may begin (weight prefetch) while the kernel in
     // front of it in the stream drains.  KAIO_B200_PDL=0 restores plain stream serialisation.

@@ -67,3 +67,33 @@ def test_qkv_decode_capture_after_warming_many_rows(oracle):
         torch.cuda.synchronize()
     for got, (w, s) in zip(o, ws):
         assert max_rel(host(got)[:m * n].reshape(m, n), oracle.qkv_int4(x[:m * k], w, s, m, n, k)) < 1e-3
+
+
+def test_qkv_scales_written_by_the_launch_in_front():
+    """The decode GEMM in front lets its dependents start before it is done; its f16 output is the QKV call's
+    scale matrix.  Back to back and with a synchronisation in between: the same bits."""
+    n, k, k0 = 512, 1024, 4096
+    g = torch.Generator(device="cuda").manual_seed(5)
+
+    def words(rows, cols):
+        return torch.randint(-2**31, 2**31 - 1, (rows // 8 * cols,), generator=g, device="cuda", dtype=torch.int32)
+
+    w0, s0 = words(k0, n), torch.full((k0 // G * n,), 0.01, device="cuda").half()
+    ws = [words(k, n) for _ in range(3)]
+    x = torch.randn(8 * k, generator=g, device="cuda").half()
+    a = [torch.rand(k // G * k0, generator=g, device="cuda").mul_(0.01).half() for _ in range(8)]
+    scales = [torch.zeros(k // G * n, device="cuda", dtype=torch.float16) for _ in range(3)]
+
+    def run(i, sync):
+        o = [torch.zeros(8 * n, device="cuda", dtype=torch.float16) for _ in range(3)]
+        torch.cuda.synchronize()
+        for j, s in enumerate(scales):
+            ops.matmul_int4(device(), a[(i + j) % 8], w0, s0, s, k // G, n, k0, G)
+        if sync:
+            torch.cuda.synchronize()
+        ops.qkv_project_int4(device(), x, *ws, *scales, *o, 8, n, k, G)
+        return torch.cat(o)
+
+    want = [run(i, True) for i in range(8)]
+    for i in range(64):
+        assert torch.equal(run(i % 8, False), want[i % 8])
