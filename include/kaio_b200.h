@@ -25,7 +25,9 @@
  *     calls on different streams may overlap; it grows on demand with cudaFree + cudaMalloc,
  *     which synchronises the device.  Growth is refused (KAIO_B200_ERR_INVALID_CONFIG) while the
  *     stream is being captured into a CUDA graph, and a graph captured earlier keeps the old
- *     address: run every op once at its largest shape before capturing;
+ *     address: run every op once at each shape that will be captured (a smaller shape may need more
+ *     scratch than a larger one; a W4A16 call of more than 16 rows leaves the scratch of calls of up to
+ *     16 rows on the same weights behind);
  *   - kaio_b200_matmul_int4 and its f16, all-gather, peer-partial and no-alloc forms with m <= 16 are
  *     launched with programmatic stream serialisation and read b_packed and scales (nothing else) without
  *     waiting for the kernel directly in front on the stream.  A kernel in front that writes these two and

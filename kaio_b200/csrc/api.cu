@@ -207,14 +207,14 @@ static StreamScratch* scratch_for(DeviceCtx* c, cudaStream_t stream)
 // Growing a scratch block frees the old one with cudaFree, which waits for the work in flight
 // on the device, and allocates: neither is allowed while the stream is being captured into a
 // CUDA graph, and a graph captured earlier keeps the old address.  So growth during a capture
-// is refused; callers warm every op at its largest shape before they capture.
+// is refused; callers run every op once at the shapes that they will capture.
 static int32_t refuse_growth_in_capture(cudaStream_t stream, const char* what)
 {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone)
         return fail(KAIO_B200_ERR_INVALID_CONFIG,
                     "%s would have to be allocated while the stream is being captured; run the op "
-                    "once at its largest shape before capturing",
+                    "once at this shape before capturing",
                     what);
     return KAIO_B200_OK;
 }
@@ -260,11 +260,14 @@ static int32_t ensure_workspace(DeviceCtx* c, cudaStream_t stream, size_t bytes,
     return KAIO_B200_OK;
 }
 
-// A fused QKV call of many rows leaves the split-K scratch of the same projections' decode step behind,
-// so that warming the op at its largest shape still covers a decode step captured later.  Not during a
-// capture, and a failure is the later call's to report.
-static void prepare_decode_scratch(DeviceCtx* c, cudaStream_t stream, int num_probs, uint32_t n)
+// A W4A16 call of many rows leaves the split-K scratch of the same weights' decode step behind (5 MB a
+// stream), whichever kernel serves it, so that warming the op with a prompt covers a decode step captured
+// later.  Not during a capture, and a failure is the later call's to report.
+static void prepare_decode_scratch(DeviceCtx* c, cudaStream_t stream, const __half* x, const DqProblem* probs,
+                                   int num_probs, uint32_t n, uint32_t k)
 {
+    if (!w4a16_decode_ok(x, probs, num_probs, 1, n, k))
+        return;
     StreamScratch* sc = scratch_for(c, stream);
     const size_t bytes = w4a16_decode_workspace_bytes(*c), counters = w4a16_decode_num_counters(num_probs, n);
     if (bytes <= sc->workspace_bytes && counters <= sc->num_tile_counters)
@@ -579,6 +582,7 @@ static int32_t run_int4(const kaio_f16* a, size_t a_len, const uint32_t* b, size
                                           sc->tile_counters, s),
                       "matmul_int4", "w4a16_decode_splitk");
     }
+    prepare_decode_scratch(ctx, s, x, &pr, 1, n, k);
     if (m <= fused_max_m() && w4a16_fused_ok(x, &pr, 1, m, n, k)) {
         const size_t ws = w4a16_fused_workspace_bytes(*ctx, 1, m, n, k);
         if (ws && (rc = ensure_workspace(ctx, s, ws, w4a16_fused_num_counters(*ctx, 1, m, n, k), &sc)))
@@ -621,6 +625,8 @@ static int32_t run_qkv(int wfmt, const char* op, const __half* x, DqProblem prob
                                           sc->tile_counters, s),
                       op, "qkv_w4a16_decode_splitk");
     }
+    if (wfmt == WFMT_S4_PACKED && !post_scale)
+        prepare_decode_scratch(ctx, s, x, probs, 3, n, k);
     if (wfmt == WFMT_S4_PACKED && !post_scale && m <= fused_max_m() &&
         w4a16_fused_ok(x, probs, 3, m, n, k)) {
         const size_t ws = w4a16_fused_workspace_bytes(*ctx, 3, m, n, k);
@@ -634,8 +640,6 @@ static int32_t run_qkv(int wfmt, const char* op, const __half* x, DqProblem prob
     if (wfmt == WFMT_S8_ROWMAJOR && post_scale && m <= w8a16_fused_max_m() &&
         w8a16_fused_ok(x, probs, 3, m, n, k))
         return finish(launch_w8a16_fused(*ctx, x, probs, 3, m, n, k, s), op, "qkv_w8a16_fused");
-    if (wfmt == WFMT_S4_PACKED && w4a16_decode_ok(x, probs, 3, 1, n, k))
-        prepare_decode_scratch(ctx, s, 3, n);
     if (dq_gemm_fast_path_ok(wfmt, x, probs, 3, true, m, n, k)) {
         if ((rc = ensure_dq_workspace(ctx, s, dq_gemm_workspace_bytes(3, n, k), &sc)))
             return rc;
@@ -1227,6 +1231,7 @@ KAIO_API int32_t kaio_b200_matmul_int4_silu_gate(const kaio_f16* x, size_t x_len
     if (!small_m && m > 128 && (uintptr_t)act % 16 == 0 &&
         dq_gemm_fast_path_ok(WFMT_S4_PACKED, xh, &pr, 1, true, m, n, k)) {
         StreamScratch* sc = nullptr;
+        prepare_decode_scratch(ctx, s, xh, &pr, 1, n, k);
         if ((rc = ensure_dq_workspace(ctx, s, dq_gemm_workspace_bytes(1, n, k), &sc)))
             return rc;
         return finish(launch_dq_gemm(*ctx, WFMT_S4_PACKED, xh, &pr, 1, true, false, m, n, k,
@@ -1345,6 +1350,7 @@ static int32_t run_int4_allgather(const char* op, const kaio_f16* a, size_t a_le
                                           sc->tile_counters, s, &copies),
                       op, "w4a16_decode_splitk_allgather");
     }
+    prepare_decode_scratch(ctx, s, x, &pr, 1, n_loc, k);
     if (m <= fused_max_m() && w4a16_fused_ok(x, &pr, 1, m, n_loc, k)) {
         const size_t ws = w4a16_fused_workspace_bytes(*ctx, 1, m, n_loc, k);
         if (ws && (rc = ensure_workspace(ctx, s, ws, w4a16_fused_num_counters(*ctx, 1, m, n_loc, k), &sc)))
@@ -1505,6 +1511,7 @@ KAIO_API int32_t kaio_b200_matmul_int4_peer_partials(const kaio_f16* a, size_t a
                                           sc->tile_counters, s, &copies),
                       op, "w4a16_decode_splitk_peer_partials");
     }
+    prepare_decode_scratch(ctx, s, x, &pr, 1, n, k);
     if (m <= fused_max_m() && w4a16_fused_ok(x, &pr, 1, m, n, k)) {
         const size_t ws = w4a16_fused_workspace_bytes(*ctx, 1, m, n, k);
         if (ws && (rc = ensure_workspace(ctx, s, ws, w4a16_fused_num_counters(*ctx, 1, m, n, k), &sc)))

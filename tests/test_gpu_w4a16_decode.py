@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from kaio_b200 import ops
+from kaio_b200 import _lib, ops
 from helpers import dev, device, host, max_rel
 
 pytestmark = pytest.mark.gpu
@@ -97,3 +97,32 @@ def test_qkv_scales_written_by_the_launch_in_front():
     want = [run(i, True) for i in range(8)]
     for i in range(64):
         assert torch.equal(run(i % 8, False), want[i % 8])
+
+
+@pytest.mark.parametrize("warm", [17, 64, 256, 512, 600])
+def test_decode_capture_after_warming_any_row_count(oracle, warm):
+    """Whichever kernel served the many rows (none of these needs split-K scratch for itself)."""
+    n, k, m = 256, 512, 4
+    rng = np.random.default_rng(warm)
+    ws, x = [weights(oracle, rng, k, n) for _ in range(3)], rng.standard_normal(warm * k).astype(np.float16)
+    wd, sd, xd = [dev(w) for w, _ in ws], [dev(s) for _, s in ws], dev(x)
+    o = [torch.zeros(warm * n, device="cuda", dtype=torch.float16) for _ in range(3)]
+    c = torch.zeros(warm * n, device="cuda")
+    # torch hands out pooled streams: one with no scratch of its own yet is what the promise is about
+    for run, outs in ((lambda rows: ops.matmul_int4(device(), xd, wd[0], sd[0], c, rows, n, k, G), [c]),
+                      (lambda rows: ops.qkv_project_int4(device(), xd, *wd, *sd, *o, rows, n, k, G), o)):
+        torch.cuda.synchronize()
+        _lib.load().kaio_b200_shutdown()
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            run(warm)
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph, stream=stream):
+                run(m)
+            for t in outs:
+                t.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+        for got, (w, s) in zip(outs, ws):
+            want = oracle.matmul_int4(x[:m * k], w, s, m, n, k) if outs[0] is c else oracle.qkv_int4(x[:m * k], w, s, m, n, k)
+            assert max_rel(host(got)[:m * n].reshape(m, n), want) < 1e-3
