@@ -252,9 +252,11 @@ static int32_t ensure_workspace(DeviceCtx* c, cudaStream_t stream, size_t bytes,
         cudaError_t err = cudaMalloc(&sc->tile_counters, counters * sizeof(uint32_t));
         if (err != cudaSuccess)
             return fail_cuda(err, "cudaMalloc(counters)");
-        err = cudaMemset(sc->tile_counters, 0, counters * sizeof(uint32_t));
+        // on the stream whose launches count with them: a non-blocking stream does not wait for the
+        // legacy stream that cudaMemset uses
+        err = cudaMemsetAsync(sc->tile_counters, 0, counters * sizeof(uint32_t), stream);
         if (err != cudaSuccess)
-            return fail_cuda(err, "cudaMemset(counters)");
+            return fail_cuda(err, "cudaMemsetAsync(counters)");
         sc->num_tile_counters = counters;
     }
     return KAIO_B200_OK;
