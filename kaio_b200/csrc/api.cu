@@ -933,10 +933,10 @@ KAIO_API int32_t kaio_b200_qkv_project_w8a8(
                                                     m, k, s);
     if (err != cudaSuccess)
         return fail_cuda(err, op);
-    // Up to 128 rows of projections of at most 64 columns and 512 k keep the CUDA-core kernel: that route
-    // is pinned by the operation's tests, not by time (us, 64 rows, K = 64 / 512: 11.8 / 52 there, 6.8 /
-    // 7.5 on the pair kernel).  Beyond, it loses by far: 725 against 22 us for 16 x 4096 x 4096.
-    bool fast = (m > 128 || n > 64 || k > 512) && (n % 16 == 0);
+    // The pair kernel wherever TMA reads the operands: few rows leave most of a tile empty, but the CUDA-core
+    // kernel is slower even for the smallest call (us a call with its quantiser, 1 x 16 x 32: 10.3 against 16.5,
+    // 128 x 64 x 512: 12.4 against 59.5, 16 x 4096 x 4096: 22 against 725).
+    bool fast = n % 16 == 0;
     for (int i = 0; i < 3; ++i)
         fast = fast && ((uintptr_t)w[i] % 16 == 0) && ((uintptr_t)out[i] % 16 == 0) &&
                ((uintptr_t)col[i] % 16 == 0);

@@ -45,7 +45,28 @@ def test_matches_the_oracle_bit_for_bit(oracle, m, n, k, seed):
     ws = [rng.integers(-127, 128, k * n, dtype=np.int8) for _ in range(3)]
     scales = [rng.uniform(0.001, 0.01, n).astype(np.float32) for _ in range(3)]
     variant = run(oracle, m, n, k, x, ws, scales)
-    assert variant == ("qkv_w8a8_tcgen05_2cta" if m > 128 and n % 16 == 0 else "qkv_w8a8_generic")
+    assert variant == "qkv_w8a8_tcgen05_2cta"
+
+
+@pytest.mark.parametrize("m,n,k,misaligned", [(64, 8, 128, None), (33, 70, 96, None), (300, 24, 64, None),
+                                              (64, 32, 128, "w"), (40, 64, 64, "out"), (129, 48, 160, "scale")])
+def test_what_tma_cannot_read_takes_the_generic_kernel(oracle, m, n, k, misaligned):
+    """N that is no multiple of 16, and buffers that do not start on 16 bytes: bit for bit as well."""
+    rng = np.random.default_rng(m + n + k)
+    x = rng.standard_normal(m * k).astype(np.float16)
+    ws = [rng.integers(-127, 128, k * n, dtype=np.int8) for _ in range(3)]
+    scales = [rng.uniform(0.001, 0.01, n).astype(np.float32) for _ in range(3)]
+
+    def put(arr, what):
+        t = dev(arr)
+        return torch.cat([t[:1], t])[1:] if what == misaligned else t
+
+    o = [put(np.full(m * n, np.nan, np.float16), "out") for _ in range(3)]
+    ops.qkv_project_w8a8(device(), dev(x), *[put(w, "w") for w in ws], *[put(s, "scale") for s in scales], *o, m, n, k)
+    assert ops.last_variant() == "qkv_w8a8_generic"
+    for t, w, s in zip(o, ws, scales):
+        want = oracle.qkv_w8a8(x, w, s, m, n, k)
+        assert np.array_equal(host(t, (m, n)).view(np.uint16), want.view(np.uint16))
 
 
 def test_projections_are_not_mixed_up(oracle):
