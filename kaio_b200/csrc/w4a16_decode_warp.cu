@@ -432,9 +432,12 @@ __global__ void __launch_bounds__(NUM_THREADS, CTAS_PER_SM) w4a16_decode_warp_ke
 
 // Column tiles of 64 (four 16-column sub-tiles per activation fragment) where every warp still gets
 // four units or more, else of 32: the activations a warp reads through L1 weigh as much as the
-// weights at M = 16 and 64 columns, and half a unit per warp is lost at the end of a launch.
-static uint32_t tile_cols(const DeviceCtx& ctx, uint32_t num_probs, uint32_t n, uint32_t k)
+// weights at M = 16 and 64 columns, and half a unit per warp is lost at the end of a launch.  One matrix of
+// that size with more than eight rows is the tcgen05 form's (see use_tc), unless it has next to no columns.
+static uint32_t tile_cols(const DeviceCtx& ctx, uint32_t num_probs, uint32_t m, uint32_t n, uint32_t k)
 {
+    if (num_probs == 1 && m > 8)
+        return MIN_TILE;
     const uint64_t units = (uint64_t)num_probs * ((n + MAX_TILE - 1) / MAX_TILE) * (k / UNIT_K);
     return units >= (uint64_t)ctx.num_sms * CTAS_PER_SM * WARPS * 4 ? MAX_TILE : MIN_TILE;
 }
@@ -504,7 +507,7 @@ cudaError_t launch_w4a16_decode(const DeviceCtx& ctx, const __half* x, const DqP
     p.m = m;
     p.n = n;
     p.k = k;
-    const uint32_t tile = tile_cols(ctx, num_probs, n, k);
+    const uint32_t tile = tile_cols(ctx, num_probs, m, n, k);
     p.num_kb = k / UNIT_K;
     p.tiles = (n + tile - 1) / tile;
     const uint32_t units = num_probs * p.tiles * p.num_kb;
@@ -553,9 +556,8 @@ cudaError_t launch_w4a16_decode(const DeviceCtx& ctx, const __half* x, const DqP
         return out_f16 ? go(w4a16_decode_warp_kernel<2, 1, true>, 2, 1)
                        : go(w4a16_decode_warp_kernel<2, 1, false>, 2, 1);
     }
-    if (wide)
-        return out_f16 ? go(w4a16_decode_warp_kernel<4, 2, true>, 4, 2)
-                       : go(w4a16_decode_warp_kernel<4, 2, false>, 4, 2);
+    if (wide)  // three matrices: f16 outputs
+        return go(w4a16_decode_warp_kernel<4, 2, true>, 4, 2);
     return out_f16 ? go(w4a16_decode_warp_kernel<2, 2, true>, 2, 2)
                    : go(w4a16_decode_warp_kernel<2, 2, false>, 2, 2);
 }

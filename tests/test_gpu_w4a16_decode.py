@@ -126,3 +126,37 @@ def test_decode_capture_after_warming_any_row_count(oracle, warm):
         for got, (w, s) in zip(outs, ws):
             want = oracle.matmul_int4(x[:m * k], w, s, m, n, k) if outs[0] is c else oracle.qkv_int4(x[:m * k], w, s, m, n, k)
             assert max_rel(host(got)[:m * n].reshape(m, n), want) < 1e-3
+
+
+@pytest.mark.parametrize("m", [1, 9, 16])
+def test_qkv_of_64_column_tiles(oracle, m):
+    """Three matrices large enough for the wide tiles, of a width that ends inside one; every third row."""
+    n, k = 5128, 5120
+    rng = np.random.default_rng(m)
+    ws, x = [weights(oracle, rng, k, n) for _ in range(3)], rng.standard_normal(m * k).astype(np.float16)
+    got = []
+    for _ in range(2):
+        o = [torch.full((m * n,), float("nan"), device="cuda", dtype=torch.float16) for _ in range(3)]
+        ops.qkv_project_int4(device(), dev(x), *[dev(w) for w, _ in ws], *[dev(s) for _, s in ws], *o, m, n, k, G)
+        got.append([host(t, (m, n)) for t in o])
+    rows = list(range(0, m, 3)) + [m - 1]
+    xs = np.ascontiguousarray(x.reshape(m, k)[rows]).reshape(-1)
+    for first, again, (w, s) in zip(*got, ws):
+        assert np.array_equal(first.view(np.uint16), again.view(np.uint16))
+        assert max_rel(first[rows], oracle.qkv_int4(xs, w, s, len(rows), n, k)) < 1e-3
+
+
+@pytest.mark.parametrize("m", [1, 8])
+def test_f16_output_of_64_column_tiles(oracle, m):
+    n, k = 14344, 8192
+    rng = np.random.default_rng(m)
+    (packed, scales), a = weights(oracle, rng, k, n), rng.standard_normal(m * k).astype(np.float16)
+    got = []
+    for _ in range(2):
+        c = torch.full((m * n,), float("nan"), device="cuda", dtype=torch.float16)
+        ops.matmul_int4(device(), dev(a), dev(packed), dev(scales), c, m, n, k, G)
+        got.append(host(c, (m, n)))
+    assert np.array_equal(got[0].view(np.uint16), got[1].view(np.uint16))
+    # f32 sums narrowed once: half a unit in the last place of f16 beside the f32 bar
+    want = oracle.matmul_int4(a, packed, scales, m, n, k).reshape(m, n).astype(np.float64)
+    assert np.all(np.abs(got[0] - want) <= 2.0 ** -11 * np.abs(want) + 1e-3 * np.maximum(np.abs(want), 1.0))
