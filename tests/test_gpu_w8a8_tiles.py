@@ -1,12 +1,18 @@
 """W8A8 over the tile widths: halves and quarters of the pair kernel's tiles, the 64- / 128- / 256-column
 tiles of the single-CTA kernel, ragged last columns and rows of each, and the pair kernel with few rows
 of a fused QKV call.  s32 sums are exact and the epilogue is one or two roundings: bit for bit."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
 from kaio_b200 import ops
 from helpers import dev, device, host
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +42,51 @@ def test_qkv(oracle, m, n, k):
     assert ops.device_status(device())[0] == 0
     for t, w, s in zip(o, ws, sc):
         assert np.array_equal(host(t, (m, n)).view(np.uint16), oracle.qkv_w8a8(x, w, s, m, n, k).view(np.uint16))
+
+
+FORCED = r"""
+import numpy as np, torch
+from kaio_b200 import ops
+from oracle import oracle
+oracle.build()
+d = ops.KaioDevice(0)
+dev = lambda a: torch.from_numpy(np.ascontiguousarray(a).reshape(-1)).cuda()
+# one row tile, two column tiles and a bit of every width; then pairs: several rounds, ragged in m and n
+for m, n, k in [(1, 16, 32), (100, 528, 160), (128, 592, 1056), (129, 80, 96), (600, 784, 672), (1100, 5136, 160)]:
+    rng = np.random.default_rng(m + n + k)
+    a, b = rng.integers(-128, 128, m * k, dtype=np.int8), rng.integers(-128, 128, k * n, dtype=np.int8)
+    sa, sw = rng.uniform(0.001, 0.01, m).astype(np.float32), rng.uniform(0.001, 0.01, n).astype(np.float32)
+    out, acc = torch.full((m * n,), float("nan"), device="cuda"), torch.zeros(m * n, dtype=torch.int32, device="cuda")
+    ops.matmul_int8_scaled(d, dev(a), dev(b), out, dev(sa), dev(sw), m, n, k)
+    assert ops.last_variant() == ("w8a8_tcgen05_2cta" if m > 128 else "w8a8_tcgen05")
+    assert np.array_equal(out.cpu().numpy().reshape(m, n), oracle.matmul_int8_scaled(a, b, sa, sw, m, n, k)), (m, n, k)
+    ops.matmul_int8(d, dev(a), dev(b), out, 0.001, m, n, k)
+    assert np.array_equal(out.cpu().numpy().reshape(m, n), oracle.matmul_int8(a, b, 0.001, m, n, k)), (m, n, k)
+    ops.matmul_int8_acc(d, dev(a), dev(b), acc, m, n, k)
+    want = a.reshape(m, k).astype(np.float64) @ b.reshape(k, n).astype(np.float64)  # exact: below 2^53
+    assert np.array_equal(acc.cpu().numpy().reshape(m, n), want.astype(np.int32)), (m, n, k)
+    assert ops.device_status(d)[0] == 0
+print("same bits")
+"""
+
+
+@pytest.mark.parametrize("cols,parts", [(64, 4), (128, 2), (256, 1)])
+def test_every_width_whatever_the_rule_picks(cols, parts):
+    """The widths are picked by a fitted cost, so a shape does not say which form it tests.  The tuning aids
+    force one: 64, 128 or 256 columns in the single-CTA kernel, quarters, halves or whole tiles in the pairs."""
+    env = dict(os.environ, KAIO_B200_W8A8_BN=str(cols), KAIO_B200_W8A8_PARTS=str(parts))
+    r = subprocess.run([sys.executable, "-c", FORCED], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same bits" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("m,n,k", [(100, 11008, 4096), (16, 28672, 4096)])
+def test_wide_few_rows(oracle, m, n, k):
+    """Sizes at which the rule leaves the 64-column tiles; sampled rows."""
+    rng = np.random.default_rng(m)
+    a, b = rng.integers(-128, 128, m * k, dtype=np.int8), rng.integers(-128, 128, k * n, dtype=np.int8)
+    sa, sw = rng.uniform(0.001, 0.01, m).astype(np.float32), rng.uniform(0.001, 0.01, n).astype(np.float32)
+    out = torch.full((m * n,), float("nan"), device="cuda")
+    ops.matmul_int8_scaled(device(), dev(a), dev(b), out, dev(sa), dev(sw), m, n, k)
+    rows = [0, m // 2, m - 1]
+    want = oracle.matmul_int8_scaled(np.ascontiguousarray(a.reshape(m, k)[rows]).reshape(-1), b, sa[rows], sw, 3, n, k)
+    assert np.array_equal(host(out, (m, n))[rows], want)
