@@ -98,7 +98,7 @@ def load() -> C.CDLL:
 
 
 class _Native:
-    """``kaio_b200/_native.so``, imported at the first use of one of its functions."""
+    """The extension module ``kaio_b200._native``, imported at the first use of one of its functions."""
 
     def __getattr__(self, name):
         import torch  # noqa: F401  (its libraries have to be loaded first)

@@ -5,8 +5,8 @@ cross-compiles without a GPU.  Each ``csrc/*.cu`` is compiled to an object in pa
 linked into ``kaio_b200/lib/libkaio_b200.so``; the CUDA runtime is linked statically and the
 driver API is reached through the runtime's entry-point lookup, so the library loads on a
 machine without ``libcuda.so`` (where every op then reports a CUDA error).  ``csrc/bindings.cpp``
-(the argument unpacking of ``kaio_b200.ops``) becomes the extension module ``kaio_b200/_native.so``,
-linked against that library.
+(the argument unpacking of ``kaio_b200.ops``) becomes the extension module ``kaio_b200/_native``,
+linked against that library; it is built again when the Python or the torch it was built for has changed.
 """
 from __future__ import annotations
 
@@ -23,7 +23,9 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(LIB_DIR, "libkaio_b200.so")
-NATIVE = os.path.join(HERE, "_native.so")
+# tagged with the Python ABI, so that another interpreter does not load it
+NATIVE = os.path.join(HERE, "_native" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+NATIVE_STAMP = os.path.join(OBJ_DIR, "native.txt")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -86,24 +88,47 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+NATIVE_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
+
+
+def _native_key() -> str:
+    """What the extension module depends on beside its sources."""
+    import torch
+    return "\n".join([f"torch {torch.__version__}", f"python {sysconfig.get_config_var('EXT_SUFFIX')}", *NATIVE_FLAGS])
+
+
+def native_is_current() -> bool:
+    if not os.path.exists(NATIVE) or not os.path.exists(NATIVE_STAMP):
+        return False
+    srcs = [os.path.join(CSRC, "bindings.cpp"), os.path.join(os.path.dirname(HERE), "include", "kaio_b200.h")]
+    if os.path.getmtime(NATIVE) < max(os.path.getmtime(f) for f in srcs):
+        return False
+    with open(NATIVE_STAMP) as f:
+        return f.read() == _native_key()
+
+
 def build_native(force: bool = False) -> str:
     """Compiles ``csrc/bindings.cpp`` against the installed torch and this library."""
-    import importlib.util
-    src = os.path.join(CSRC, "bindings.cpp")
-    header = os.path.join(os.path.dirname(HERE), "include", "kaio_b200.h")
-    if not force and os.path.exists(NATIVE) and \
-            os.path.getmtime(NATIVE) >= max(os.path.getmtime(src), os.path.getmtime(header)):
+    if not force and native_is_current():
         return NATIVE
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    import torch
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    untagged = os.path.join(HERE, "_native.so")
+    if untagged != NATIVE and os.path.exists(untagged):
+        os.remove(untagged)  # an earlier build's, which any Python would load
+    src = os.path.join(CSRC, "bindings.cpp")
+    torch_dir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     inc = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include/torch/csrc/api/include"),
            sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
-    r = subprocess.run([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+    r = subprocess.run([shutil.which("g++") or "g++", *NATIVE_FLAGS, f'-DKAIO_TORCH_VERSION="{torch.__version__}"',
                         *[f"-I{d}" for d in inc], src, "-o", NATIVE, f"-L{LIB_DIR}", "-lkaio_b200",
                         f"-L{os.path.join(torch_dir, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
                         "-Wl,-rpath,$ORIGIN/lib"], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on {src}:\n{r.stdout}\n{r.stderr}")
+    with open(NATIVE_STAMP, "w") as f:
+        f.write(_native_key())
     return NATIVE
 
 

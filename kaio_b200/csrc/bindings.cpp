@@ -395,6 +395,20 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, g_methods
 
 PyMODINIT_FUNC PyInit__native()
 {
+    // compiled against one torch's C++ headers; another's tensors may be laid out differently
+    PyObject* torch = PyImport_ImportModule("torch");
+    PyObject* version = torch ? PyObject_GetAttrString(torch, "__version__") : nullptr;
+    PyObject* text = version ? PyObject_Str(version) : nullptr;
+    Py_XDECREF(torch);
+    Py_XDECREF(version);
+    if (!text)
+        return nullptr;
+    const bool same = PyUnicode_CompareWithASCIIString(text, KAIO_TORCH_VERSION) == 0;
+    if (!same)
+        PyErr_Format(PyExc_ImportError, "built for torch %s, this is torch %U", KAIO_TORCH_VERSION, text);
+    Py_DECREF(text);
+    if (!same)
+        return nullptr;
     PyObject* errors = PyImport_ImportModule("kaio_b200.errors");
     if (!errors)
         return nullptr;

@@ -1,10 +1,16 @@
 """Argument handling of the native half of ``kaio_b200.ops``, as far as it shows without a GPU: what a call
 took and refused when every argument went through ctypes."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
 from kaio_b200 import ops
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def refused(exc, fn, *args, match=None):
@@ -59,3 +65,24 @@ def test_a_wrong_dtype_is_named_as_torch_names_it():
     a = torch.zeros(4, dtype=torch.int8)
     for dtype in (torch.float64, torch.bfloat16, torch.uint8, torch.int16, torch.int64, torch.bool, torch.float32):
         refused(TypeError, ops.matmul_int8, a.to(dtype), a, a, 1.0, 1, 1, 32, match=f"a: expected dtype torch.int8, got {dtype}")
+
+
+def test_the_extension_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    from kaio_b200 import build
+    for name in ("NATIVE", "NATIVE_STAMP"):
+        monkeypatch.setattr(build, name, str(tmp_path / name))
+    (tmp_path / "NATIVE").write_text("")
+    assert not build.native_is_current()  # no stamp
+    (tmp_path / "NATIVE_STAMP").write_text(build._native_key())
+    assert build.native_is_current()
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    assert not build.native_is_current()
+
+
+def test_the_extension_of_another_torch_does_not_load():
+    code = ("import torch; torch.__version__ = '0.0'\n"
+            "from kaio_b200 import ops\n"
+            "try: ops.selftest_bounded_wait(ops.KaioDevice(0), 0)\n"
+            "except RuntimeError as e: print(e)")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert "built for torch" in r.stdout and "kaio_b200.build" in r.stdout, r.stdout + r.stderr
