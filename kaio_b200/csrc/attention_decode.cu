@@ -300,7 +300,7 @@ cudaError_t launch_attention_decode(const DeviceCtx& ctx, const AttnParams& ap, 
     // each: many small CTAs even out the last wave.  With fewer pairs sixteen warps, so that eight
     // CTAs of a pair still keep enough loads in flight.  The cluster is as wide as there are blocks
     // for its warps.
-    const bool wide = pairs * 8 * 4 < (uint32_t)ctx.num_sms * 16;
+    const bool wide = (uint64_t)pairs * 8 * 4 < (uint64_t)ctx.num_sms * 16;
     const uint32_t warps = wide ? 16 : 4;
     uint32_t csize = 1;
     while (csize < 8 && csize * warps < blocks)

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from kaio_b200 import ops
+from kaio_b200 import CudaError, ops
 from helpers import assert_attention_close, dev, device, host
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +40,19 @@ def test_decode(oracle, b, h, sk, d):
 def test_decode_causal_strided_hot(oracle, d):
     run(oracle, 2, 2, 40, d, True, 2 * d + 8)       # row 0 sees key 0 only; padded rows
     run(oracle, 1, 4, 1000, d, False, 4 * d, 3.7)   # scores spread over some twenty powers of two
+
+
+def test_more_pairs_than_a_grid_has_rows():
+    """65536 (batch, head) pairs and more: the one-row kernel numbers its CTAs in one dimension; the kernels
+    for several rows do not, and such a call is refused on the host as it always was."""
+    b, sk, d = 70000, 3, 64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v = [torch.randn(b * n, d, generator=g, device="cuda").half() for n in (1, sk, sk)]
+    out = torch.zeros(b * d, device="cuda", dtype=torch.float16)
+    ops.attention_mha_f16(device(), q, k, v, out, b, 1, 1, sk, d, d, False)
+    assert ops.last_variant() == "attention_decode"
+    s = torch.einsum("bd,bsd->bs", q.float(), k.view(b, sk, d).float()) / 8.0
+    want = torch.einsum("bs,bsd->bd", torch.softmax(s, 1), v.view(b, sk, d).float())
+    assert_attention_close(host(out, (b, d)).astype(np.float32), want.cpu().numpy())
+    with pytest.raises(CudaError):
+        ops.attention_mha_f16(device(), torch.cat([q, q]), k, v, torch.cat([out, out]), b, 1, 2, sk, d, d, False)
