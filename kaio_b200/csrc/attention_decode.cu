@@ -15,8 +15,8 @@
 //  * The key range of a pair is cut over the CTAs of a cluster (and over the warps of a CTA); the
 //    partial (max, sum, output) meet in distributed shared memory.  No scratch buffer, no atomics,
 //    so the result does not depend on arrival order and a first call may be captured in a graph.
-// Measured at 8 x 32 heads, 2000 keys, d 128 (262 MB): 62.6 us with the tile kernel (4.2 TB/s), 50.9 us here (5.2 TB/s
-// of 6.65 copied); 8 heads over 8192 keys 10.8 us; head_dim 64 went to a scalar kernel before.
+// Measured at 8 x 32 heads, 2000 keys, d 128 (262 MB), per call: 66 us with the tile kernel (4.0 TB/s), 50.2 us here
+// (5.2 TB/s of 6.54 copied); 8 heads over 8192 keys 10.8 us; head_dim 64 went to a scalar kernel before.
 #include <cooperative_groups.h>
 
 #include "common.cuh"

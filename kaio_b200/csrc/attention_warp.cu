@@ -13,8 +13,8 @@
 // by 2^12 so that lo stays clear of f16's subnormals), because the scalar kernel kept it in f32.  Against
 // 64-bit arithmetic, 2-norm over head_dim 64, f32 out: 1.3e-7 (64 keys causal) to 2.6e-7 (384 keys), the scalar
 // kernel 2.2e-7 to 4.5e-7; the tcgen05 form, whose P is one f16, 1.3e-4 to 2.0e-4 at head_dim 128, here 1.5e-7 to 3.5e-7.
-// Measured: one head of 384 keys, d 128, causal: 12.3 us (tcgen05 form) -> 7.4 us; 1 x 8 heads of 128
-// keys 5.5 us (9.9 us for 300 keys on the tcgen05 form); d 64, 8 x 32 heads of 512 causal: 63 us.
+// Measured, us per call back to back: one head of 384 keys, d 128, causal: 12.3 (tcgen05 form) -> 8.2; d 64, one
+// head of 384 keys 96 (scalar kernel, alone) -> 6.3, 8 x 32 heads of 512 causal 16.6 ms -> 65 us.
 #include <cfloat>
 
 #include "common.cuh"

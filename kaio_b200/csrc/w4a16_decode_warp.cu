@@ -26,13 +26,13 @@
 // sums meet in shared memory, and where a range ends inside a tile the CTAs park f32 partials that
 // the last one to arrive adds in ascending CTA order (deterministic; no float atomics).
 // Programmatic dependent launch: what runs before griddepcontrol.wait reads only weights and scales, and of
-// three matrices not even these.  The early reads save 0.5 to 1 us where calls follow each other (13.6 against
-// 14.4 us for three of 4096 x 4096 at M = 8), but weights or scales that the kernel in front writes would be
+// three matrices not even these.  The early reads save 0.5 to 1 us where calls follow each other (13.2 against
+// 14.2 us for three of 4096 x 4096 at M = 8), but weights or scales that the kernel in front writes would be
 // read too early if it lets its dependents start; a fused QKV call never asked its callers to mind that.
-// Measured (us, tcgen05 form -> this one, weights from HBM), M = 1, K x N: 1024 x 1024 7.1 -> 2.5,
-// 4096 x 4096 13.0 -> 7.8, 28672 x 1024 28.2 -> 10.7, 4096 x 11008 15.1 -> 12.4, 8192 x 28672 41 -> 33.2
-// (3.5 TB/s); three 4096 x 4096 matrices at M = 8 62.7 (f16 copy of the weights, then a GEMM) -> 14.1.
-// Issue-bound: 25 instructions per word at 0.5 per cycle and scheduler, no pipe above 35 %.
+// Measured (us per call back to back, tcgen05 form -> this one), M = 1, K x N: 1024 x 1024 7.6 -> 2.9, 4096 x 4096
+// 13.3 -> 8.2, 4096 x 11008 15.4 -> 11.7, 8192 x 28672 41 -> 34 (3.5 TB/s); three 4096 x 4096 matrices at M = 8 63 (f16
+// copy of the weights, then a GEMM) -> 14.2.  At M = 1, 4096 x 11008: 30 instructions per word at 0.39 per cycle and
+// scheduler, no pipe above 28 %: four warps per scheduler do not cover the latencies of the chain.
 #include <cstdlib>
 
 #include "common.cuh"
@@ -122,6 +122,7 @@ __device__ __forceinline__ __half2 and_xor(uint32_t w, uint32_t mask, uint32_t f
     return *reinterpret_cast<__half2*>(&r);
 }
 
+// (The conversion by exponent bits is the published one of Kim et al., "Who Says Elephants Can't Run", 2022.)
 // Eight signed nibbles -> f16(q) * scale, rounded to f16, as the pairs (0,4) (1,5) (2,6) (3,7).  The
 // flipped sign bit makes a nibble q + 8; under the exponent of 1024 it is 1024 + (q + 8), or
 // 1024 + 16 (q + 8) where it sits four bits up.

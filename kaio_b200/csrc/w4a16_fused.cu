@@ -632,8 +632,8 @@ struct FusedPlan {
 //   rows  128     : 9.5 cycles/k (128-k stages),                                   fix-up 2560 k
 //   rows  256     : 17  cycles/k (64-k stages, dequantisation ~ tensor pipe),      fix-up 4096 k
 // More rows per tile dequantise each weight fewer times, fewer rows give more tiles to fill the
-// SMs; e.g. M = 256 runs as 256-row tiles on a whole 70B FFN matrix (224 column tiles) and as
-// 128-row tiles on one eighth of it (28 column tiles).
+// SMs; e.g. M = 256 runs as 128-row tiles spread evenly on a whole 70B FFN matrix (224 column tiles)
+// and on one eighth of it (28).  (Fitted when the epilogue still spilled; every size has gained since.)
 static FusedPlan fused_plan(const DeviceCtx& ctx, int num_probs, uint32_t m, uint32_t n, uint32_t k)
 {
     static const uint32_t kRows[4] = {32, 64, 128, 256};

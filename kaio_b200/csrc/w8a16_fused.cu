@@ -15,8 +15,9 @@
 //    activations by TMA as the K-major operand;
 //  * the K range of a tile is cut over the CTAs of a cluster while they all run at once; the partial
 //    tiles meet in distributed shared memory, in rank order: no scratch, no atomics, one launch.
-// Measured (us, three projections, weights from HBM, two launches -> this one): 2048 x 2048, M = 64:
-// 38.9 -> 12.1; 4096 x 4096, M = 300 / 512: 92 / 93 -> 60 / 66; M = 16 / 128 / 256: 23 / 30 / 36.
+// Measured (us per call, three projections, weights from HBM, two launches -> this one): 2048 x 2048, M = 64:
+// 38.9 -> 14.0; 4096 x 4096, M = 300 / 512: 92 / 93 -> 60 / 66.  The kernel alone: 12.1 and, 4096 x 4096, M = 16 /
+// 128 / 256: 23 / 30 / 36.
 #include "common.cuh"
 #include "kernels.h"
 
