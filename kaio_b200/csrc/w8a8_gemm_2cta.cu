@@ -76,8 +76,7 @@ struct Params {
     const float* w_scale[3];  // per problem
     float scale;
     uint32_t m, n, k;     // n = columns of ONE problem
-    uint32_t full_tiles;  // tiles [0, full_tiles) run whole; each later tile runs as `parts` items
-    uint32_t part_shift;  // parts = 1 << part_shift = 2 or 4
+    uint32_t full_tiles;  // tiles [0, full_tiles) run whole; each later tile runs as 1 << PART_SHIFT items
     uint32_t* status;
 };
 
@@ -90,7 +89,9 @@ struct alignas(64) TensorMaps {
     CUtensorMap c[NP];
 };
 
-template <int EPI, int NP>
+// PART_SHIFT: tiles beyond p.full_tiles run in two (1) or four (2) parts.  As a parameter of the launch it
+// cost the calls of several rounds 0.5 to 1 %.
+template <int EPI, int NP, uint32_t PART_SHIFT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 w8a8_gemm_2cta_kernel(const __grid_constant__ TensorMaps<NP> maps,
                       const __grid_constant__ Params p)
@@ -123,16 +124,16 @@ w8a8_gemm_2cta_kernel(const __grid_constant__ TensorMaps<NP> maps,
     const uint32_t num_tiles = tiles_m * tiles_n;
     const uint32_t num_kb = (p.k + BK - 1) / BK;
     // work item -> (tile, which part)
-    const uint32_t num_items = p.full_tiles + ((num_tiles - p.full_tiles) << p.part_shift);
-    const uint32_t part_cols = BN >> p.part_shift;
+    const uint32_t num_items = p.full_tiles + ((num_tiles - p.full_tiles) << PART_SHIFT);
+    constexpr uint32_t part_cols = BN >> PART_SHIFT;
     auto item_tile = [&](uint32_t item, uint32_t& tile, uint32_t& part) {
         if (item < p.full_tiles) {
             tile = item;
             part = WHOLE;
         } else {
-            const uint32_t i = (item - p.full_tiles) >> p.part_shift;
+            const uint32_t i = (item - p.full_tiles) >> PART_SHIFT;
             tile = p.full_tiles + i;
-            part = item - p.full_tiles - (i << p.part_shift);
+            part = item - p.full_tiles - (i << PART_SHIFT);
         }
     };
 
@@ -233,10 +234,10 @@ w8a8_gemm_2cta_kernel(const __grid_constant__ TensorMaps<NP> maps,
             // B rows (one per k) are 128 bytes in a whole tile, 64 or 32 bytes in a part; the shared
             // window is below 256 KB, so an address only fills its field of the descriptor
             const uint64_t b_desc0 = whole               ? make_smem_desc_sw128(0, 16, 1024)
-                                     : p.part_shift == 1 ? make_smem_desc_sw64(0, 16, 512)
+                                     : PART_SHIFT == 1 ? make_smem_desc_sw64(0, 16, 512)
                                                          : make_smem_desc_sw32(0, 16, 256);
             const uint32_t b_step = (UMMA_K * (whole ? 128u : part_cols / 2)) >> 4;
-            const uint32_t idesc = whole ? IDESC : (p.part_shift == 1 ? IDESC_HALF : IDESC_QUARTER);
+            const uint32_t idesc = whole ? IDESC : (PART_SHIFT == 1 ? IDESC_HALF : IDESC_QUARTER);
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 if (!mbar_wait_bounded_cluster(full_bar(s), ph, abort_flag, p.status, SITE_FULL,
                                                KERNEL_W8A8)) {
@@ -405,11 +406,14 @@ static bool half_tiles_disabled()
 }
 
 // How the tiles of a call are cut into items.  Part tiles stage A once per part, but fill the pairs of
-// a short last round, or of the only one, and leave less to store after the last MMA.  Nanoseconds per
-// 128 k of a round, and from the launch to the end of the stores beside them, for a whole tile, halves
-// and quarters, fitted to (us, whole / halves / quarters): 512^3 7.1 / 6.3 / 5.8, 256^3 6.8 / 5.6 / 5.0,
-// 1024^3 8.9 / 8.0 / 7.6, 512 x 4096 x 512 8.5 / 7.4 / 8.6, 1500 x 1008 x 3008 14.8 / 13.5 / 20.2,
-// 2048^3 12.5 / 17.1 / 26.0.
+// the only round and leave less to store after the last MMA.  Nanoseconds per 128 k, and from the launch to
+// the end of the stores beside them, for a whole tile, halves and quarters, fitted to (us, whole / halves /
+// quarters): 512^3 7.1 / 6.3 / 5.8, 256^3 6.8 / 5.6 / 5.0, 1024^3 8.9 / 8.0 / 7.6, 512 x 4096 x 512 8.5 / 7.4 /
+// 8.6, 1500 x 1008 x 3008 14.8 / 13.5 / 20.2, 2048^3 12.5 / 17.1 / 26.0.
+// Parts only while they all run in one round: a second round of parts waits for the stores of the first where
+// K is short, and stages A once more where it is long.  Measured over 1480 shapes (us a call, whole / halves):
+// 322 x 6560 x 64, 2048 x 2048 x 128 and 129 x 16384 x 256 10.5 / 12.6, 2048 x 4064 x 64 16.7 / 18.7; with the
+// cost per round alone one in fifteen shapes was slower in parts, with this line three of 1480 (64 columns).
 struct TileSplit {
     uint32_t full_tiles, parts;
 };
@@ -432,8 +436,8 @@ static TileSplit tile_split(uint32_t tiles, uint32_t max_pairs, uint32_t num_kb)
     }
     for (uint32_t i = 1; i <= 2; ++i) {
         const uint32_t parts = 1u << i;
-        const float cost = rounds(tiles * parts) * (float)num_kb * PER_KB[i] + FIXED[i];
-        if (forced ? forced == (int)parts : cost < best_cost) {
+        const float cost = (float)num_kb * PER_KB[i] + FIXED[i];
+        if (forced ? forced == (int)parts : tiles * parts <= max_pairs && cost < best_cost) {
             best_cost = cost;
             best = {0, parts};
         }
@@ -490,20 +494,23 @@ static cudaError_t launch_pair_kernel(const DeviceCtx& ctx, const int8_t* a,
     p.k = k;
     p.status = ctx.status;
     p.full_tiles = split.full_tiles;
-    p.part_shift = split.parts == 2 ? 1u : 2u;
     const uint32_t items = split.full_tiles + split.parts * (tiles - split.full_tiles);
     const uint32_t pairs = items < max_pairs ? items : max_pairs;
 
-    static bool attr_set[64] = {};
-    if (!attr_set[ctx.device]) {
-        err = cudaFuncSetAttribute(w8a8_gemm_2cta_kernel<EPI, NP>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (err != cudaSuccess)
-            return err;
-        attr_set[ctx.device] = true;
-    }
-    w8a8_gemm_2cta_kernel<EPI, NP><<<pairs * 2, NUM_THREADS, SMEM_BYTES, stream>>>(maps, p);
-    return cudaGetLastError();
+    auto go = [&](auto kernel, bool& attr_set) -> cudaError_t {
+        if (!attr_set) {
+            const cudaError_t e =
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+            if (e != cudaSuccess)
+                return e;
+            attr_set = true;
+        }
+        kernel<<<pairs * 2, NUM_THREADS, SMEM_BYTES, stream>>>(maps, p);
+        return cudaGetLastError();
+    };
+    static bool attr_set[2][64] = {};
+    return split.parts == 2 ? go(w8a8_gemm_2cta_kernel<EPI, NP, 1>, attr_set[0][ctx.device])
+                            : go(w8a8_gemm_2cta_kernel<EPI, NP, 2>, attr_set[1][ctx.device]);
 }
 
 cudaError_t launch_w8a8_gemm_2cta(const DeviceCtx& ctx, int epi, const int8_t* a, const int8_t* b,
