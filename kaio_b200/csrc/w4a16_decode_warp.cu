@@ -460,12 +460,37 @@ bool w4a16_decode_ok(const void* x, const DqProblem* probs, int num_probs, uint3
     return (uintptr_t)x % 16 == 0;
 }
 
-// Nine to sixteen rows double the MMAs and the activations; from 2^25 weights on the tcgen05 form is
-// then the faster one (us, tcgen05 / this one, M = 16, K x N: 4096 x 4096 13.2 / 10.5, 4096 x 11008 15.2
-// / 17.2, 8192 x 28672 41.2 / 48.2).  Three matrices in one launch are this kernel's alone.
-static bool use_tc(int num_probs, uint32_t m, uint32_t n, uint32_t k)
+// Where the tcgen05 form, which always served one matrix before, is the faster one (us back to back, tcgen05 /
+// this one; three matrices in one launch are this kernel's alone):
+//  * a tile of one or two units of K, whatever the rows: most of a CTA's warps idle at every tile's end.  M = 1 / 16:
+//    4096 x 128 3.9 / 8.2, 4.1 / 11.9; 28672 x 256 4.7 / 5.9, 4.9 / 8.6 (N x K); from 128 columns on;
+//  * few units in all, so a CTA takes eight, and K no power of two of units: every tile is cut and summed through
+//    memory.  4096 columns, K = 384 / 640 at M = 1: 6.1 / 8.2, 0.90 of it; K = 384 .. 1280 at M = 16: 0.67 to 0.96;
+//  * more than eight rows, which double the MMAs and the activations, over many columns: the line follows
+//    rows * columns^2 * K.  M = 16: 16384 x 1024 10.0 / 11.7, 28672 x 1024 12.1 / 14.7, 9216 x 2048 10.4 / 11.3, 11008 x
+//    4096 15.2 / 17.1, 28672 x 8192 41.9 / 53.5; below it 16384 x 512 7.4 / 5.7, 11008 x 1024 11.7 / 9.6, 4096 x 8192
+//    15.1 / 13.9, 2048 x 28672 23.4 / 18.2; M = 9: 28672 x 1024 11.8 / 13.3, 8192 x 2048 10.4 / 10.2; up to 8192
+//    columns a little later: 8192 x 2560 14.1 / 11.9, x 3072 12.5 / 12.7;
+//  * very many columns: 98304 x 512 at M = 1 0.73 of this one's time, at M = 16 0.54; from K = 1792 on alike at M = 1.
+// Over 337 widths and depths at M = 1, 8, 9 and 16 the pick is 0.4 % off the better form on
+// average, 12.8 % with the line at 2^25 weights and nine rows alone.
+static bool use_tc(const DeviceCtx& ctx, int num_probs, uint32_t m, uint32_t n, uint32_t k)
 {
-    return num_probs == 1 && m > 8 && (uint64_t)n * k >= (1u << 25);
+    using namespace w4dw;
+    if (num_probs != 1 || n < 128)
+        return false;
+    const uint32_t kb = k / UNIT_K;
+    if (kb <= 2)
+        return true;
+    const uint64_t tiles = (n + MIN_TILE - 1) / MIN_TILE, max_grid = (uint64_t)ctx.num_sms * CTAS_PER_SM;
+    const bool cut = n >= 256 && 8 % kb != 0 && kb % 8 != 0 && tiles * kb <= max_grid * WARPS;
+    if (m <= 8)
+        return (cut && kb <= 5) || (n >= 49152 && kb <= 12);
+    if ((cut && kb <= 10) || n >= 49152)
+        return true;
+    if (tiles % max_grid == 0)  // no tile is cut here: 9472 columns, K = 1536 at M = 16 9.8 / 6.3
+        return (uint64_t)n * k >= (1u << 25);
+    return (kb >= 7 || n >= 24576) && (double)m * n * n * k > (n > 8192 ? 2.2e12 : 2.9e12);
 }
 
 size_t w4a16_decode_workspace_bytes(const DeviceCtx& ctx)
@@ -487,7 +512,7 @@ cudaError_t launch_w4a16_decode(const DeviceCtx& ctx, const __half* x, const DqP
                                 const OutputCopies* copies)
 {
     using namespace w4dw;
-    if (use_tc(num_probs, m, n, k))
+    if (use_tc(ctx, num_probs, m, n, k))
         return launch_w4a16_decode_tc(ctx, x, probs[0], out_f16, m, n, k, workspace, counters, stream,
                                       copies);
     Params p;

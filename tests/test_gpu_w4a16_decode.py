@@ -160,3 +160,19 @@ def test_f16_output_of_64_column_tiles(oracle, m):
     # f32 sums narrowed once: half a unit in the last place of f16 beside the f32 bar
     want = oracle.matmul_int4(a, packed, scales, m, n, k).reshape(m, n).astype(np.float64)
     assert np.all(np.abs(got[0] - want) <= 2.0 ** -11 * np.abs(want) + 1e-3 * np.maximum(np.abs(want), 1.0))
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(127, 128), (128, 128), (130, 256), (255, 384), (256, 384), (1000, 640), (520, 1280),
+                                 (16384, 1024), (49160, 384)])
+def test_on_both_sides_of_the_line_between_the_two_forms(oracle, m, n, k):
+    rng = np.random.default_rng(m * 7 + n + k)
+    (packed, scales), a = weights(oracle, rng, k, n), rng.standard_normal(m * k).astype(np.float16)
+    got = []
+    for _ in range(2):
+        c = torch.full((m * n,), float("nan"), device="cuda")
+        ops.matmul_int4(device(), dev(a), dev(packed), dev(scales), c, m, n, k, G)
+        got.append(host(c, (m, n)))
+    assert ops.device_status(device())[0] == 0
+    assert np.array_equal(got[0], got[1])
+    assert max_rel(got[0], oracle.matmul_int4(a, packed, scales, m, n, k)) < 1e-3
